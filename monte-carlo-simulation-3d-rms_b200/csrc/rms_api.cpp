@@ -77,7 +77,7 @@ struct rms_device_state {
     int device = -1;
     cudaStream_t own = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
-    DevBuf labels, packed, axons, wavef, tables, tablesf, slots, sig_slots, vscr, qtab, bvec, grad, gpair, ev_step,
+    DevBuf labels, packed, axons, wavef, tables, rows, slots, sig_slots, vscr, qtab, bvec, grad, gpair, ev_step,
         ev_pair, ev_coef, out, out_sig, err, tr_init, tr_vox, tr_ev, tr_pos, adj_g, adj_sums, adj_dwave, adj_ck, adj_ws, adj_blist, adj_bcount, adj_xbin, adj_ajw, adj_wq,
         stage, counts;
     HostPinned h_out, h_axons;
@@ -87,7 +87,7 @@ struct rms_device_state {
 
     ~rms_device_state() {
         if (device >= 0) cudaSetDevice(device);
-        for (DevBuf* b : {&labels, &packed, &axons, &wavef, &tables, &tablesf, &slots, &sig_slots, &vscr, &qtab, &bvec, &grad,
+        for (DevBuf* b : {&labels, &packed, &axons, &wavef, &tables, &rows, &slots, &sig_slots, &vscr, &qtab, &bvec, &grad,
                           &gpair, &ev_step, &ev_pair, &ev_coef, &out, &out_sig, &err, &tr_init,
                           &tr_vox, &tr_ev, &tr_pos, &adj_g, &adj_sums, &adj_dwave, &adj_ck, &adj_ws, &adj_blist,
                           &adj_bcount, &adj_xbin, &adj_ajw, &adj_wq, &stage, &counts})
@@ -491,6 +491,14 @@ int prepare_lattice(rms_sim* s, cudaStream_t st, bool split, int bits) {
     return RMS_OK;
 }
 
+// Row sets of an axon walked by `warps` warps at once (a row set is row_sz
+// doubles): warps of one row set add into the same addresses at about the same
+// time, so one set per 64 warps, at most 16, and no more than 256 MB of them.
+int split_row_sets(int64_t warps, size_t row_sz) {
+    const int64_t fit = std::max<int64_t>(1, (int64_t)(((size_t)256 << 20) / (row_sz * sizeof(double))));
+    return (int)std::max<int64_t>(1, std::min<int64_t>({warps / 64, 16, fit}));
+}
+
 // Settings every simulation of one split launch must share (the signal
 // tables and the record schedule are the launch's).
 bool same_schedule(const rms_sim* a, const rms_sim* b) {
@@ -510,7 +518,7 @@ struct LaunchPlan {
     cudaStream_t st = nullptr;
     int prec = 0, grid = 0, block = 0, variant = 0, bits = 8, naxons = 0, T = 0, nb = 0, ngrad = 0,
         ngrad_pad = 0, nvals = 0, nseg = 0;
-    size_t row = 0, nrow = 0, nsig = 0;
+    size_t row = 0, nrow = 0, nsig = 0, nsets = 0;   // doubles: one axon's results, all, signals, row sets
     bool multi = false, has_sig = false, wavemode = false;
     int64_t trace_n = 0;
     std::vector<AxonDesc> axons;
@@ -581,15 +589,20 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
     // signal row: PGSE, one value per gradient; waveforms, (cos, sin) per waveform
     const int ngrad = wavemode ? 2 * s->nwave : s->ngrad();
     const int ngrad_pad = std::max(32, ((ngrad + 31) / 32) * 32);
-    const size_t row = (size_t)T * nvals;
 
-    const int nseg = nwarps;   // one accumulator row set per warp
+    const int nseg = nwarps;   // COMPAT: one accumulator row set per warp
     // The SPLIT walk runs in the table form (axon fields and seeds from device
-    // memory, tiles from a queue, each warp's rows added into the axon totals
+    // memory, tiles from a queue, records added into a few row sets per axon
     // with FP64 atomics): for one axon too, where it is 1.3x faster than the
     // form reading kernel parameters (fewer registers), at the price of sums
     // repeatable only up to their order.  COMPAT: per-warp rows, ordered sum.
     const bool multi = prec == RMS_PREC_SPLIT;
+    // one axon's results: COMPAT the summed rows, SPLIT its fields (gather_rows_kernel)
+    const size_t row = multi ? (size_t)T * (kColCount + nc_max + nb) : (size_t)T * nvals;
+    // SPLIT row sets: moments [kRowHead][tpad], then signals [T][nb_pad]
+    const int tpad = (T + 7) / 8 * 8, nb_pad = nvals - kRowHead;
+    const size_t row_sz = (size_t)kRowHead * tpad + (size_t)T * nb_pad;
+    size_t nsets = 0;
 
     // inputs
     for (LaunchJob& j : jobs) {
@@ -619,18 +632,24 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
     }
     if (prec == RMS_PREC_SPLIT) {
         p.axons.resize(naxons);
-        for (int k = 0; k < naxons; ++k)
-            fill_axon_desc(p.axons[k], jobs[k].s, jobs[k].w0, jobs[k].w1, tile_begin[k], jobs[k].seed,
+        for (int k = 0; k < naxons; ++k) {
+            AxonDesc& x = p.axons[k];
+            fill_axon_desc(x, jobs[k].s, jobs[k].w0, jobs[k].w1, tile_begin[k], jobs[k].seed,
                            jobs[k].s->dev->packed.as<uint8_t>());
+            x.ncopy = split_row_sets(std::min<int64_t>(tile_begin[k + 1] - tile_begin[k], nwarps), row_sz);
+            x.row_off = (int64_t)nsets;
+            nsets += (size_t)x.ncopy * row_sz;
+        }
         RMS_CUDA(d->axons.ensure(sizeof(AxonDesc) * naxons));
     }
 
     // accumulators
-    RMS_CUDA(d->slots.ensure((size_t)nseg * row * sizeof(double)));
+    if (multi) RMS_CUDA(d->rows.ensure(nsets * sizeof(double)));
+    else RMS_CUDA(d->slots.ensure((size_t)nseg * row * sizeof(double)));
     RMS_CUDA(d->out.ensure((size_t)naxons * row * sizeof(double)));
     RMS_CUDA(d->err.ensure(16));   // error word, then the multi-axon tile counter at byte 8
     if (has_sig) {
-        RMS_CUDA(d->sig_slots.ensure((size_t)nseg * ngrad_pad * sizeof(double)));
+        if (!multi) RMS_CUDA(d->sig_slots.ensure((size_t)nseg * ngrad_pad * sizeof(double)));
         RMS_CUDA(d->out_sig.ensure((size_t)naxons * ngrad_pad * sizeof(double)));
         const size_t per_thread = wavemode ? (size_t)s->nwave : (size_t)s->npairs * 3;
         RMS_CUDA(d->vscr.ensure(std::max<size_t>(per_thread * nthr * sizeof(double), 16)));
@@ -681,7 +700,10 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
     a.traj = traj;
     a.traj_split = (o && o->traj_split) ? 1 : 0;
     a.traj_n = jobs[0].w1 - jobs[0].w0;
-    a.out_rows = d->out.as<double>();
+    a.rows = d->rows.as<double>();
+    a.tpad = tpad;
+    a.nb_pad = nb_pad;
+    a.row_sz = row_sz;
     a.out_sig = d->out_sig.as<double>();
     if (!p.axons.empty()) a.axon0 = p.axons[0];
     a.trace_n = trace_n;
@@ -690,7 +712,7 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
 
     p.d = d; p.st = st; p.prec = prec; p.grid = grid; p.block = block; p.variant = variant; p.bits = lattice_bits;
     p.naxons = naxons; p.T = T; p.nb = nb; p.ngrad = ngrad; p.ngrad_pad = ngrad_pad; p.nvals = nvals; p.nseg = nseg;
-    p.row = row; p.nrow = nrow; p.nsig = nsig; p.multi = multi; p.has_sig = has_sig; p.wavemode = wavemode;
+    p.row = row; p.nrow = nrow; p.nsig = nsig; p.nsets = nsets; p.multi = multi; p.has_sig = has_sig; p.wavemode = wavemode;
     p.trace_n = trace_n;
     return RMS_OK;
 }
@@ -704,19 +726,22 @@ int enqueue_launch(LaunchPlan& p, rms_sim* s, bool events) {
     const WalkArgs& a = p.a;
     if (p.prec == RMS_PREC_SPLIT)
         RMS_CUDA(cudaMemcpyAsync(d->axons.p, d->h_axons.p, sizeof(AxonDesc) * p.naxons, cudaMemcpyHostToDevice, st));
-    RMS_CUDA(cudaMemsetAsync(d->slots.p, 0, (size_t)p.nseg * p.row * sizeof(double), st));
-    if (p.multi) RMS_CUDA(cudaMemsetAsync(d->out.p, 0, p.nrow * sizeof(double), st));
+    if (p.multi) RMS_CUDA(cudaMemsetAsync(d->rows.p, 0, p.nsets * sizeof(double), st));
+    else RMS_CUDA(cudaMemsetAsync(d->slots.p, 0, (size_t)p.nseg * p.row * sizeof(double), st));
     RMS_CUDA(cudaMemsetAsync(d->err.p, 0, 16, st));
     if (p.has_sig) {
-        RMS_CUDA(cudaMemsetAsync(d->sig_slots.p, 0, (size_t)p.nseg * p.ngrad_pad * sizeof(double), st));
         if (p.multi) RMS_CUDA(cudaMemsetAsync(d->out_sig.p, 0, p.nsig * sizeof(double), st));
+        else RMS_CUDA(cudaMemsetAsync(d->sig_slots.p, 0, (size_t)p.nseg * p.ngrad_pad * sizeof(double), st));
     }
     if (events) RMS_CUDA(cudaEventRecord(d->e0, st));
     int e = (p.prec == RMS_PREC_COMPAT) ? launch_walk_compat(a, p.grid, p.block, p.trace_n > 0, st)
                                         : launch_walk_split(a, p.bits, p.variant, p.grid, st);
     if (e) return cuda_fail((cudaError_t)e, "walk kernel launch");
     if (events) RMS_CUDA(cudaEventRecord(d->e1, st));
-    if (!p.multi) {
+    if (p.multi) {
+        e = launch_gather_rows(a, d->out.as<double>(), p.row, st);
+        if (e) return cuda_fail((cudaError_t)e, "row gather launch");
+    } else {
         // COMPAT: the warps' rows summed in a fixed order (repeatable)
         e = launch_reduce_slots(a.slots, p.nseg, p.row, d->out.as<double>(), st);
         if (!e && p.has_sig)
@@ -764,25 +789,38 @@ int finish_launch(std::vector<LaunchJob>& jobs, LaunchPlan& p, bool events) {
         ms_run = ms_walk;
     }
 
-    // unpack record rows into the reference's field layouts
+    // the results into the reference's field layouts: SPLIT fields lie as they
+    // are, COMPAT record rows are taken apart
     const int T = p.T, nb = p.nb, ngrad = p.ngrad;
     for (int k = 0; k < p.naxons; ++k) {
         rms_sim* sk = jobs[k].s;
         const double* hk = h + (size_t)k * p.row;
         const int nc = sk->nc;
-        sk->sig0.assign(T, 0.0);
-        sk->dx2.assign((size_t)T * 6, 0.0);
-        sk->dx4.assign((size_t)T * 15, 0.0);
-        sk->npar_count.assign((size_t)T * nc, 0.0);
-        sk->sigre.assign((size_t)T * nb, 0.0);
-        for (int t = 0; t < T; ++t) {
-            const double* r = hk + (size_t)t * p.nvals;
-            sk->sig0[t] = r[kColSig0];
-            for (int q = 0; q < 6; ++q) sk->dx2[t * 6 + q] = r[kColDx2 + q];
-            for (int q = 0; q < 15; ++q) sk->dx4[t * 15 + q] = r[kColDx4 + q];
-            for (int c = 0; c < nc; ++c) sk->npar_count[t * nc + c] = r[kColCount + c];
-            if (sk->mode == RMS_MODE_NARROW)
-                for (int q = 0; q < nb; ++q) sk->sigre[(size_t)t * nb + q] = r[kRowHead + q];
+        if (p.multi) {
+            auto take = [&hk](std::vector<double>& v, size_t n) {
+                v.assign(hk, hk + n);
+                hk += n;
+            };
+            take(sk->sig0, T);
+            take(sk->dx2, (size_t)T * 6);
+            take(sk->dx4, (size_t)T * 15);
+            take(sk->npar_count, (size_t)T * nc);
+            take(sk->sigre, (size_t)T * nb);
+        } else {
+            sk->sig0.assign(T, 0.0);
+            sk->dx2.assign((size_t)T * 6, 0.0);
+            sk->dx4.assign((size_t)T * 15, 0.0);
+            sk->npar_count.assign((size_t)T * nc, 0.0);
+            sk->sigre.assign((size_t)T * nb, 0.0);
+            for (int t = 0; t < T; ++t) {
+                const double* r = hk + (size_t)t * p.nvals;
+                sk->sig0[t] = r[kColSig0];
+                for (int q = 0; q < 6; ++q) sk->dx2[t * 6 + q] = r[kColDx2 + q];
+                for (int q = 0; q < 15; ++q) sk->dx4[t * 15 + q] = r[kColDx4 + q];
+                for (int c = 0; c < nc; ++c) sk->npar_count[t * nc + c] = r[kColCount + c];
+                if (sk->mode == RMS_MODE_NARROW)
+                    for (int q = 0; q < nb; ++q) sk->sigre[(size_t)t * nb + q] = r[kRowHead + q];
+            }
         }
         sk->sig.assign(sk->mode == RMS_MODE_PGSE ? ngrad : 0, 0.0);
         for (int q = 0; q < (int)sk->sig.size(); ++q) sk->sig[q] = h[p.nrow + (size_t)k * p.ngrad_pad + q];
@@ -867,7 +905,7 @@ namespace {
 
 std::vector<const void*> graph_buffers(const rms_graph* g) {
     const rms_device_state* d = g->plan.d;
-    std::vector<const void*> v{d->axons.p, d->slots.p, d->out.p, d->err.p, d->sig_slots.p, d->out_sig.p,
+    std::vector<const void*> v{d->axons.p, d->rows.p, d->slots.p, d->out.p, d->err.p, d->sig_slots.p, d->out_sig.p,
                                d->vscr.p, d->tables.p, d->qtab.p, d->bvec.p, d->grad.p, d->gpair.p,
                                d->ev_step.p, d->ev_pair.p, d->ev_coef.p, d->wavef.p, d->h_out.p, d->h_axons.p};
     for (const LaunchJob& j : g->jobs) v.push_back(j.s->dev ? j.s->dev->packed.p : nullptr);

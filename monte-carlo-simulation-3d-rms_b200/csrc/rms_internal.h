@@ -28,7 +28,9 @@ struct AxonDesc {
     int s0, s1;                 // padded lattice strides: (n2+2)(n3+2), n3+2
     int64_t walker_begin, walker_end;   // walker ids (random streams) within the axon's job
     int64_t tile_begin;
+    int64_t row_off;            // its first row set, doubles into WalkArgs::rows
     uint64_t seed;
+    int ncopy;                  // its row sets (split_row_sets)
     float res;
     int same_cross;             // same-label faces always crossed, compartment 0 never entered
     int flight;                 // free flight allowed (same_cross and nite >= 4)
@@ -71,12 +73,16 @@ struct WalkArgs {
     int* err;                   // device error word (kErr* bits), zeroed per run
     unsigned long long* tile_ctr;   // table-form launches: next tile to hand out, zeroed per run
     int table_form;             // walk even one axon from the axon table (what a graph replay rewrites)
-    // split launches: the axons and their tiles; with several axons each warp
-    // adds its rows into out_rows[axon][timepoints][nvals] / out_sig[axon][ngrad_pad]
+    // split launches: the axons and their tiles; the table form adds records
+    // into row sets of row_sz doubles, moments [kRowHead][tpad] then signals
+    // [timepoints][nb_pad], axon k's ncopy of them from its row_off on, and
+    // signals into out_sig[axon][ngrad_pad]
     const AxonDesc* axons;
     int naxons;
     int64_t ntiles;
-    double* out_rows;
+    double* rows;
+    int tpad, nb_pad;
+    size_t row_sz;
     double* out_sig;
     // general waveforms: phase per um of a bin's displacement sum (waveform x
     // dt), [bin][waveform][axis]; optional per-walker bin means out,
@@ -99,9 +105,12 @@ struct WalkArgs {
 // Launchers (rms_walk_*.cu, rms_reduce.cu).  All asynchronous on `stream`;
 // they return a cudaError_t value (0 = success).
 int launch_walk_compat(const WalkArgs& a, int grid, int block, bool trace, void* stream);
-// Split walk over a.naxons axons (a.axons, a.ntiles, per-warp a.slots, and
-// a.out_rows/out_sig for several axons); lattice_bits: packed lattice format.
+// Split walk over a.naxons axons (a.axons, a.ntiles, and a.rows/out_sig, or the
+// no-allocation form's per-warp a.slots); lattice_bits: packed lattice format.
 int launch_walk_split(const WalkArgs& a, int lattice_bits, int variant, int grid, void* stream);
+// The table form's totals: axon k's fields into out + k * fields, each axon's
+// row sets added up (sig0 [T], dx2 [T][6], dx4 [T][15], counts [T][nc], signals [T][nbvec]).
+int launch_gather_rows(const WalkArgs& a, double* out, size_t fields, void* stream);
 int split_variant_count();
 bool split_variant_walks(int variant, int mode, int rule);   // variants past the first: narrow/PGSE, reflecting
 int split_variant_block(int variant);   // threads per block of a launch variant

@@ -29,10 +29,10 @@
 //    hardware sine/cosine and reciprocal for the direction and face times;
 //  - per-walker sums that grow over the walk (T2 exponent, PGSE displacement
 //    sums) are carried in FP32 for at most 32 steps and folded into FP64;
-//  - cross-walker sums: FP32 products per walker, staged in shared memory and
-//    summed per column over the warp in FP64, per-warp FP64 rows, added into
-//    each axon's totals with FP64 atomics (the no-allocation walk: an ordered
-//    FP64 reduction, rms_reduce.cu).
+//  - cross-walker sums: records staged in shared memory, and every few records
+//    the FP32 products of a warp's walkers summed in FP64 and added with FP64
+//    atomics into a few row sets per axon, which a last pass adds up (the
+//    no-allocation walk: per-warp rows and an ordered reduction, rms_reduce.cu).
 //
 // Mirror walls: the reference mirrors the origin image at the end of a step
 // for each wall the step touched (main.cu:302-310).  A step shorter than a
@@ -46,6 +46,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
+
+#include <algorithm>
 
 #include "philox.cuh"
 #include "rms_internal.h"
@@ -63,28 +65,6 @@ struct SplitVariant { int block, minb; };
 constexpr int kLeapCap = 64;   // equal-step-length leap: tries per step before staying put
 constexpr SplitVariant kVariants[] = {{256, 4}, {256, 3}, {256, 2}, {128, 8}, {512, 2}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-
-// Add a warp's accumulator rows (and PGSE signal row) into axon `axon`'s
-// totals and clear them (multi-axon launches; other warps add concurrently).
-__device__ __noinline__ void flush_rows(double* slot, double* sig_slot, double* out, double* os, size_t n,
-                                        int ngrad, int lane) {
-    for (size_t i = lane; i < n; i += 32) {
-        const double x = slot[i];
-        if (x != 0.0) {
-            atomicAdd(out + i, x);
-            slot[i] = 0.0;
-        }
-    }
-    if (os) {
-        for (int i = lane; i < ngrad; i += 32) {
-            const double x = sig_slot[i];
-            if (x != 0.0) {
-                atomicAdd(os + i, x);
-                sig_slot[i] = 0.0;
-            }
-        }
-    }
-}
 
 // General waveforms, at the end of bin `bin`: X (voxels) is the bin's
 // displacement sum; every waveform's phase gets wave_b . X res, and the bin's
@@ -115,8 +95,17 @@ __device__ __noinline__ void wave_bin(const double* __restrict__ wave, int nwave
     }
 }
 
+// A value into the totals: the no-allocation walk's rows are the warp's own
+// (a plain add, summed in order afterwards), every other launch's are shared.
+template <bool ONE>
+__device__ __forceinline__ void add_out(double* p, double x) {
+    if (ONE) *p += x;
+    else atomicAdd(p, x);
+}
+
 // General waveforms, after the last step: the warp's sums of s0 cos(phase) and
 // s0 sin(phase) per waveform, (cos, sin) pairs into the signal row.
+template <bool ONE>
 __device__ __noinline__ void wave_final(const double* ph, int nthr, int nwave, double s0, double* sig_slot,
                                         int lane) {
     for (int base = 0; base < 2 * nwave; base += 32) {
@@ -131,55 +120,154 @@ __device__ __noinline__ void wave_final(const double* ph, int nthr, int nwave, d
             if (lane == k) mine = rc;
             if (lane == k + 1) mine = rs;
         }
-        if (lane < cnt) sig_slot[base + lane] += mine;
+        if (lane < cnt) add_out<ONE>(sig_slot + base + lane, mine);
     }
 }
 
-// A record of the warp's 32 walkers added into the warp's row (row layout of
-// rms_internal.h): each lane stages its 22 moments [sig0, dx2 x6, dx4 x15]
-// (FP32 products) in shared memory, and lane c < 22 adds column c over the 32
-// walkers in FP64, in lane order (four interleaved partials, combined in a
-// fixed order); lanes 22.. take the compartment counts (integer warp sums).
-// KC columns per pass.  Not inlined: the step loop keeps its registers (the
-// inlined form cost the batch walk ~3 % more time).
-template <int KC>
-__device__ __noinline__ void record_row(double* row, float s0, float dx, float dy, float dz, int ai, bool active,
-                                        int lane, float (*stage)[KC + 1]) {
-    const float xx = dx * dx, yy = dy * dy, zz = dz * dz;
-    const float sxx = s0 * xx, syy = s0 * yy, szz = s0 * zz;
-    const float mv[22] = {s0,      sxx,          s0 * dx * dy, s0 * dx * dz, syy,
-                          s0 * dy * dz, szz,     sxx * xx,     sxx * dx * dy, sxx * dx * dz,
-                          sxx * yy, sxx * dy * dz, sxx * zz,   syy * dx * dy, syy * dx * dz,
-                          szz * dx * dy, szz * dx * dz, syy * yy, syy * dy * dz, syy * zz,
-                          szz * dy * dz, szz * zz};
-    double r = 0.0;
+// Records are taken in batches of KR: at a record every lane stages its
+// walker's displacement and T2 weight in shared memory, and every KR
+// records the warp adds the batch up.  With KR = 8, lane (r, g) = (lane % 8,
+// lane / 8) sums six of record r's 22 moments [sig0, dx2 x6, dx4 x15] over the
+// 32 walkers (FP32 products, FP64 sums): group g holds the six second-order
+// products of A = s0, s0 x^2, s0 y^2 or s0 z^2, which are dx2 and, each once,
+// dx4 (of the products that two groups could form one keeps its own column);
+// the spare one of group 2 is sig0.  KR = 4 halves the walkers between two
+// lanes.  A staged row is 4 x 32 floats and 4 of padding, so the 16-byte loads
+// of KR lanes (four walkers of KR records) cover all banks.
+//
+// Why batches: one record at a time cost 32 shared loads, 32 FP32 -> FP64
+// conversions (a 16-per-clock pipe), 32 FP64 adds and 22 stores per warp with
+// one lane per column, and 10 warp reductions for the counts; here a
+// warp-record costs five loads, 24 conversions and adds and ~30 paired products
+// (__fmul2_rn: two walkers an instruction), no shuffle.  1e6 walkers x 2000
+// steps on a 128x128x900 axon, walk kernel: 12.5 / 35.6 ms with 100 / 2000
+// records before, 12.3 / 27.1 ms now.  KR = 8 up to 256 threads a block (4.2 KB
+// of staging per warp), 4 above, so the static shared memory stays under 48 KB.
+__host__ __device__ constexpr int rec_batch(int block) { return block <= 256 ? 8 : 4; }
+constexpr int kStageRow = 4 * 32 + 4;   // floats of a staged record: x, y, z, s0 of 32 walkers, and 4 of padding
+constexpr int kStageOnes = -4;          // before the first record, four ones
+
+// Where the sums go.  ONE: the warp's own rows [timepoint][nvals] (plain adds).
+// Otherwise one of the axon's ncopy row sets, moments as [column][tpad] so that
+// the KR records of a batch are neighbours, by fire-and-forget FP64 atomics in
+// L2: a few row sets shared by all warps stay in L2 and need neither a row set
+// per warp (1.2 GB for 1000 records, cleared and streamed through HBM) nor a
+// flush when a warp moves on to another axon.
+template <int KR, bool ONE>
+__device__ __noinline__ void add_moments(const float* st, const unsigned* msk, double* dst, int stride, int nrec,
+                                         unsigned act, int nc, int lane) {
+    constexpr int NW = 4 * KR;   // walkers per lane
+    const int r = lane & (KR - 1), g = (lane / KR) & 3, half = lane / (4 * KR);
+    __syncwarp();
+    double q0 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0, q4 = 0.0, q5 = 0.0;
+    const float* row_st = st + r * kStageRow + half * NW;
+    // the group's m with A = s0 m^2: ones, x, y or z
+    const float* mp = g == 0 ? st + kStageOnes : row_st + (g - 1) * 32;
+    const int minc = g == 0 ? 0 : 4;
+#pragma unroll 1
+    for (int k = 0; k < NW; k += 4, mp += minc) {
+        const float4 X = *reinterpret_cast<const float4*>(row_st + k), Y = *reinterpret_cast<const float4*>(row_st + 32 + k),
+                     Z = *reinterpret_cast<const float4*>(row_st + 64 + k),
+                     S = *reinterpret_cast<const float4*>(row_st + 96 + k), M = *reinterpret_cast<const float4*>(mp);
 #pragma unroll
-    for (int pass = 0; pass < 22 / KC; ++pass) {
-        __syncwarp();
-#pragma unroll
-        for (int c = 0; c < KC; ++c) stage[lane][c] = mv[pass * KC + c];
-        __syncwarp();
-        const int col = lane - pass * KC;
-        if (col >= 0 && col < KC) {
-            double q0 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0;
-#pragma unroll
-            for (int l = 0; l < 32; l += 4) {
-                q0 += (double)stage[l][col];
-                q1 += (double)stage[l + 1][col];
-                q2 += (double)stage[l + 2][col];
-                q3 += (double)stage[l + 3][col];
-            }
-            r = (q0 + q1) + (q2 + q3);
+        for (int h = 0; h < 2; ++h) {
+            // two walkers at a time (paired FP32 products)
+            const float2 x = h ? make_float2(X.z, X.w) : make_float2(X.x, X.y);
+            const float2 y = h ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y);
+            const float2 z = h ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y);
+            const float2 s0 = h ? make_float2(S.z, S.w) : make_float2(S.x, S.y);
+            const float2 m = h ? make_float2(M.z, M.w) : make_float2(M.x, M.y);
+            const float2 A = __fmul2_rn(s0, __fmul2_rn(m, m)), Ax = __fmul2_rn(A, x);
+            const float2 p0 = __fmul2_rn(A, __fmul2_rn(x, x)), p1 = __fmul2_rn(Ax, y), p2 = __fmul2_rn(Ax, z),
+                         p3 = __fmul2_rn(A, __fmul2_rn(y, y)), p4 = __fmul2_rn(__fmul2_rn(A, y), z),
+                         p5 = __fmul2_rn(A, __fmul2_rn(z, z));
+            q0 += (double)(g == 2 ? s0.x : p0.x); q0 += (double)(g == 2 ? s0.y : p0.y);
+            q1 += (double)p1.x; q1 += (double)p1.y;
+            q2 += (double)p2.x; q2 += (double)p2.y;
+            q3 += (double)p3.x; q3 += (double)p3.y;
+            q4 += (double)p4.x; q4 += (double)p4.y;
+            q5 += (double)p5.x; q5 += (double)p5.y;
         }
     }
-    unsigned cnt = 0u;
-#pragma unroll
-    for (int c = 0; c < 10; ++c) {
-        const unsigned n = __reduce_add_sync(0xffffffffu, (active && ai == c) ? 1u : 0u);
-        if (lane == kColCount + c) cnt = n;
+    if (NW < 32) {
+        q0 += __shfl_xor_sync(0xffffffffu, q0, 16); q1 += __shfl_xor_sync(0xffffffffu, q1, 16);
+        q2 += __shfl_xor_sync(0xffffffffu, q2, 16); q3 += __shfl_xor_sync(0xffffffffu, q3, 16);
+        q4 += __shfl_xor_sync(0xffffffffu, q4, 16); q5 += __shfl_xor_sync(0xffffffffu, q5, 16);
     }
-    if (lane >= kColCount) r = (double)cnt;
-    row[lane] += r;
+    if (r >= nrec || half) return;
+    double* row = ONE ? dst + (size_t)r * stride : dst + r;
+    const size_t cs = ONE ? 1 : (size_t)stride;
+    // columns of the group's six products (-1: another group's)
+    const int c0 = g == 0 ? 1 : (g == 1 ? 7 : (g == 2 ? 0 : -1));
+    const int c1 = g == 0 ? 2 : (g == 1 ? 8 : (g == 2 ? 13 : 15));
+    const int c3 = g == 0 ? 4 : (g == 1 ? 10 : (g == 2 ? 17 : -1));
+    const int c4 = g == 0 ? 5 : (g == 1 ? 11 : (g == 2 ? 18 : 20));
+    if (c0 >= 0) add_out<ONE>(row + c0 * cs, q0);
+    add_out<ONE>(row + c1 * cs, q1);
+    add_out<ONE>(row + (c1 + 1) * cs, q2);
+    if (c3 >= 0) add_out<ONE>(row + c3 * cs, q3);
+    add_out<ONE>(row + c4 * cs, q4);
+    add_out<ONE>(row + (c4 + 1) * cs, q5);
+    // compartment counts from the staged label bits
+    const unsigned m0 = msk[3 * r], m1 = msk[3 * r + 1], m2 = msk[3 * r + 2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int c = 2 * g + k;
+        const int cnt = __popc(act & ((c & 1) ? m0 : ~m0) & ((c & 2) ? m1 : ~m1) & ((c & 4) ? m2 : ~m2));
+        if (c < nc && cnt) add_out<ONE>(row + (kColCount + c) * cs, (double)cnt);
+    }
+}
+
+// The batch's narrow-pulse signals: lane j holds b-value base + j and adds
+// s0 cos(q n.dx) over the tile's walkers, read as broadcasts from the staged
+// rows -- one cosine, one conversion and one FP64 add per walker and b-value.
+// One b-value at a time over the 32 lanes took 10 shuffles and 5 FP64 adds more.
+template <bool ONE>
+__device__ __noinline__ void add_signals(const float* st, const double* __restrict__ qtab,
+                                         const double* __restrict__ bvec, int nb, double* dst, int stride, int nrec,
+                                         int nw, int lane) {
+    __syncwarp();
+    for (int base = 0; base < nb; base += 32) {
+        const int jb = base + lane;
+        const bool in = jb < nb;
+        const float bx = in ? (float)__ldg(bvec + jb * 3) : 0.0f, by = in ? (float)__ldg(bvec + jb * 3 + 1) : 0.0f,
+                    bz = in ? (float)__ldg(bvec + jb * 3 + 2) : 0.0f;
+        for (int r = 0; r < nrec; ++r) {
+            const float q = in ? (float)__ldg(qtab + (size_t)r * nb + jb) : 0.0f;
+            double s = 0.0;
+#pragma unroll 4
+            for (int w = 0; w < nw; ++w) {
+                const float* v = st + r * kStageRow + w;
+                const float qx = q * (v[0] * bx + v[32] * by + v[64] * bz);
+                s += (double)(v[96] * cosf(qx));
+            }
+            if (in) add_out<ONE>(dst + (size_t)r * stride + jb, s);
+        }
+    }
+}
+
+constexpr int kPark = 22;
+__device__ __forceinline__ void park_walker(volatile uint32_t* p, const SplitWalker& w, const DomainStream& perm,
+                                            float q0, float q1, float q2, float q3) {
+    p[0] = w.lin; p[1] = w.cell;
+    p[2] = __float_as_uint(w.o0); p[3] = __float_as_uint(w.o1); p[4] = __float_as_uint(w.o2);
+    p[5] = (uint32_t)w.D0; p[6] = (uint32_t)w.D1; p[7] = (uint32_t)w.D2;
+    p[8] = __float_as_uint(w.Fm0); p[9] = __float_as_uint(w.Fm1); p[10] = __float_as_uint(w.Fm2);
+    p[11] = (uint32_t)w.ai; p[12] = __float_as_uint(w.cur_step); p[13] = __float_as_uint(w.cur_k);
+    p[14] = __float_as_uint(w.w32);
+    p[15] = perm.q1; p[16] = perm.q2; p[17] = perm.q3;
+    p[18] = __float_as_uint(q0); p[19] = __float_as_uint(q1); p[20] = __float_as_uint(q2); p[21] = __float_as_uint(q3);
+}
+__device__ __forceinline__ void unpark_walker(const volatile uint32_t* p, SplitWalker& w, DomainStream& perm,
+                                              float& q0, float& q1, float& q2, float& q3) {
+    w.lin = p[0]; w.cell = p[1];
+    w.o0 = __uint_as_float(p[2]); w.o1 = __uint_as_float(p[3]); w.o2 = __uint_as_float(p[4]);
+    w.D0 = (int)p[5]; w.D1 = (int)p[6]; w.D2 = (int)p[7];
+    w.Fm0 = __uint_as_float(p[8]); w.Fm1 = __uint_as_float(p[9]); w.Fm2 = __uint_as_float(p[10]);
+    w.ai = (int)p[11]; w.cur_step = __uint_as_float(p[12]); w.cur_k = __uint_as_float(p[13]);
+    w.w32 = __uint_as_float(p[14]);
+    perm.q1 = p[15]; perm.q2 = p[16]; perm.q3 = p[17];
+    q0 = __uint_as_float(p[18]); q1 = __uint_as_float(p[19]); q2 = __uint_as_float(p[20]); q3 = __uint_as_float(p[21]);
 }
 
 // ONE: the no-allocation walk's form -- one axon, whose scalars are read from
@@ -190,13 +278,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
     // of path, Pij and the step-length ratio that rescales the rest of a step
     constexpr int kTab = 2 * NCMAX + 2 * NCMAX * NCMAX;
     __shared__ float s_tab[BLOCK / 32][kTab];
-    // per warp, a record's 22 moments of its 32 walkers, staged for the column
-    // sums (all 22 at once up to 256 threads a block, else in two halves: the
-    // static shared memory stays under 48 KB a block)
-    constexpr int kCols = BLOCK <= 256 ? 22 : 11;
-    __shared__ float s_stage[BLOCK / 32][32][kCols + 1];
+    // per warp, a batch of records of its 32 walkers (add_moments) and the
+    // bits of their labels
+    constexpr int KR = rec_batch(BLOCK);
+    __shared__ __align__(16) float s_stage[BLOCK / 32][4 + KR * kStageRow];
+    __shared__ unsigned s_mask[BLOCK / 32][KR * 3];
 
     const int lane = threadIdx.x & 31;
+    if (lane < 4) s_stage[threadIdx.x >> 5][lane] = 1.0f;   // kStageOnes
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
     const int warp_global = gtid >> 5;
@@ -208,18 +297,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
     constexpr bool sums = pgse || wave;   // displacement sums over the walk
     const bool mirror = (a.boundary == 0);
 
-    // A warp keeps its rows for its current axon and, in the table form, adds
-    // them into that axon's totals (FP64 atomics) when it moves on to another
-    // axon or finishes.  ONE (the no-allocation walk) keeps one row set per
-    // warp, summed in order afterwards.
     int ax = 0;          // current axon
-    int held = -1;       // axon whose records the warp's rows hold
+    int held = -1;       // axon whose tables the warp holds
     int64_t next_tb = ONE ? INT64_MAX : ((a.naxons > 1) ? a.axons[1].tile_begin : INT64_MAX);
     // a field of the current axon: kernel parameters for ONE, else the axon
     // table (read where used, so it holds no registers)
 #define AXF(f) (ONE ? a.axon0.f : a.axons[ax].f)
-    double* slot = a.slots + (size_t)warp_global * a.timepoints * a.nvals;
-    double* sig_slot = sums ? a.sig_slots + (size_t)warp_global * a.ngrad_pad : nullptr;
 
     // The table form (every SPLIT launch but the no-allocation walk, one axon
     // or many): a queue (one counter per launch) hands out tiles in order, so
@@ -240,10 +323,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
             }
         }
         if (held != ax) {
-            if (!ONE && held >= 0)
-                flush_rows(slot, sig_slot, a.out_rows + (size_t)held * a.timepoints * a.nvals,
-                           sums ? a.out_sig + (size_t)held * a.ngrad_pad : nullptr,
-                           (size_t)a.timepoints * a.nvals, a.ngrad, lane);   // previous axon's records to its totals
             held = ax;
             // this axon's tables into the warp's shared memory
             __syncwarp();
@@ -387,68 +466,104 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                     } while (evi < a.nevents && a.ev_step[evi] == i + 1);
                     next_ev = (evi < a.nevents) ? a.ev_step[evi] : -1;
                 }
-                if (i == a.tn - 1 && wave) {
-                    wave_final(a.vscr + gtid, nthr, a.nwave, active ? exp(-(w64 + (double)wk.w32)) : 0.0, sig_slot, lane);
-                } else if (i == a.tn - 1) {
-                    // final T2-weighted signal: phase_j = |g| (g_hat . V) res dt
-                    const double s0 = active ? exp(-(w64 + (double)wk.w32)) : 0.0;
-                    const double scale = a.res * a.dt;
-                    for (int base = 0; base < a.ngrad; base += 32) {
-                        double mine = 0.0;
-                        const int cnt = min(32, a.ngrad - base);
-                        for (int k = 0; k < cnt; ++k) {
-                            const int jg = base + k;
-                            const double* vv = a.vscr + (size_t)(a.gpair[jg] * 3) * nthr + gtid;
-                            const double* g = a.grad + 6 * jg;
-                            const double phase =
-                                g[2] * (vv[0] * g[3] + vv[nthr] * g[4] + vv[2 * (size_t)nthr] * g[5]) * scale;
-                            const double r = warp_sum(s0 * cos(phase));
-                            if (lane == k) mine = r;
-                        }
-                        if (lane < cnt) sig_slot[base + lane] += mine;
-                    }
-                }
             }
 
             if (i == next_rec) {
-                const int tidx = rec++;
-                next_rec += a.tstep;
-                if (tidx < a.timepoints) {
-                    w64 += (double)wk.w32;
-                    wk.w32 = 0.0f;
-                    const float s0 = active ? expf(-(float)w64) : 0.0f;
-                    const float res = AXF(res);
-                    const float dx = ((float)D0 + (o0 - Fm0)) * res;
-                    const float dy = ((float)D1 + (o1 - Fm1)) * res;
-                    const float dz = ((float)D2 + (o2 - Fm2)) * res;
-                    double* row = slot + (size_t)tidx * a.nvals;
-                    record_row<kCols>(row, s0, dx, dy, dz, wk.ai, active, lane, s_stage[threadIdx.x >> 5]);
-                    if (!sums) {
-                        for (int base = 0; base < a.nbvec; base += 32) {
-                            double mine = 0.0;
-                            const int cnt = min(32, a.nbvec - base);
-                            for (int k = 0; k < cnt; ++k) {
-                                const int jb = base + k;
-                                const float q = (float)a.qtab[(size_t)tidx * a.nbvec + jb];
-                                const float qx = q * (dx * (float)a.bvec[jb * 3 + 0] + dy * (float)a.bvec[jb * 3 + 1] +
-                                                      dz * (float)a.bvec[jb * 3 + 2]);
-                                const double rr = warp_sum((double)(s0 * cosf(qx)));
-                                if (lane == k) mine = rr;
-                            }
-                            if (lane < cnt) row[kRowHead + base + lane] += mine;
-                        }
+                const int r = rec & (KR - 1), rec0 = rec - r;   // slot in the batch, the batch's first record
+                ++rec;
+                next_rec = rec < a.timepoints ? next_rec + a.tstep : -1;
+                w64 += (double)wk.w32;
+                wk.w32 = 0.0f;
+                const float s0 = active ? expf(-(float)w64) : 0.0f;
+                const float res = AXF(res);
+                const float dx = ((float)D0 + (o0 - Fm0)) * res;
+                const float dy = ((float)D1 + (o1 - Fm1)) * res;
+                const float dz = ((float)D2 + (o2 - Fm2)) * res;
+                float* st = s_stage[threadIdx.x >> 5] + 4;
+                unsigned* msk = s_mask[threadIdx.x >> 5];
+                float* mine = st + r * kStageRow + lane;
+                mine[0] = dx; mine[32] = dy; mine[64] = dz; mine[96] = s0;
+                const unsigned b0 = __ballot_sync(0xffffffffu, wk.ai & 1), b1 = __ballot_sync(0xffffffffu, wk.ai & 2),
+                               b2 = __ballot_sync(0xffffffffu, wk.ai & 4);
+                if (lane < 3) msk[3 * r + lane] = lane == 0 ? b0 : (lane == 1 ? b1 : b2);
+                if (r == KR - 1 || rec == a.timepoints) {
+                    // the batch's sums into the totals (a warp's own rows, or one
+                    // of the axon's row sets); the walker waits in local memory
+                    // meanwhile, its registers are the sums' (left to itself the
+                    // compiler keeps part of it there through the step loop)
+                    volatile uint32_t park[kPark];
+                    park_walker(park, wk, perm, q0, q1, q2, q3);
+                    const unsigned act = __ballot_sync(0xffffffffu, active);
+                    double* set = ONE ? a.slots + (size_t)warp_global * a.timepoints * a.nvals
+                                      : a.rows + AXF(row_off) + (size_t)(warp_global % AXF(ncopy)) * a.row_sz;
+                    add_moments<KR, ONE>(st, msk, ONE ? set + (size_t)rec0 * a.nvals : set + rec0,
+                                         ONE ? a.nvals : a.tpad, rec - rec0, act, AXF(nc), lane);
+                    if (!sums && a.nbvec > 0)
+                        add_signals<ONE>(st, a.qtab + (size_t)rec0 * a.nbvec, a.bvec, a.nbvec,
+                                         ONE ? set + (size_t)rec0 * a.nvals + kRowHead
+                                             : set + (size_t)kRowHead * a.tpad + (size_t)rec0 * a.nb_pad,
+                                         ONE ? a.nvals : a.nb_pad, rec - rec0, 32, lane);
+                    __syncwarp();
+                    unpark_walker(park, wk, perm, q0, q1, q2, q3);
+                }
+            }
+        }
+        if (sums) {
+            double* sig_slot = ONE ? a.sig_slots + (size_t)warp_global * a.ngrad_pad
+                                   : a.out_sig + (size_t)ax * a.ngrad_pad;
+            if (wave) {
+                wave_final<ONE>(a.vscr + gtid, nthr, a.nwave, active ? exp(-(w64 + (double)wk.w32)) : 0.0, sig_slot, lane);
+            } else {
+                // final T2-weighted signal: phase_j = |g| (g_hat . V) res dt
+                const double s0 = active ? exp(-(w64 + (double)wk.w32)) : 0.0;
+                const double scale = a.res * a.dt;
+                for (int base = 0; base < a.ngrad; base += 32) {
+                    double mine = 0.0;
+                    const int cnt = min(32, a.ngrad - base);
+                    for (int k = 0; k < cnt; ++k) {
+                        const int jg = base + k;
+                        const double* vv = a.vscr + (size_t)(a.gpair[jg] * 3) * nthr + gtid;
+                        const double* g = a.grad + 6 * jg;
+                        const double phase =
+                            g[2] * (vv[0] * g[3] + vv[nthr] * g[4] + vv[2 * (size_t)nthr] * g[5]) * scale;
+                        const double r = warp_sum(s0 * cos(phase));
+                        if (lane == k) mine = r;
                     }
+                    if (lane < cnt) add_out<ONE>(sig_slot + base + lane, mine);
                 }
             }
         }
     }
-    if (!ONE && held >= 0)
-        flush_rows(slot, sig_slot, a.out_rows + (size_t)held * a.timepoints * a.nvals,
-                   sums ? a.out_sig + (size_t)held * a.ngrad_pad : nullptr, (size_t)a.timepoints * a.nvals, a.ngrad,
-                   lane);
 }
 
 #undef AXF
+
+// Totals of every axon from its row sets, in the result fields' layout: axon
+// k's block of `fields` doubles holds sig0 [T], dx2 [T][6], dx4 [T][15], counts
+// [T][nc] and signals [T][nbvec], so the host copies each field as it lies.
+__global__ void gather_rows_kernel(const WalkArgs a, double* __restrict__ out, size_t fields) {
+    const AxonDesc* x = a.axons + blockIdx.y;
+    const int T = a.timepoints, nc = x->nc, ncopy = x->ncopy;
+    const double* src = a.rows + x->row_off;
+    double* dst = out + (size_t)blockIdx.y * fields;
+    const size_t n = (size_t)T * (kColCount + nc + a.nbvec);
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+        // element e of the block -> (record, column) of the row sets
+        size_t at;
+        const size_t uT = (size_t)T;
+        if (e < uT) at = e;
+        else if (e < 7 * uT) { const size_t i = e - uT; at = (1 + i % 6) * a.tpad + i / 6; }
+        else if (e < 22 * uT) { const size_t i = e - 7 * uT; at = (7 + i % 15) * a.tpad + i / 15; }
+        else if (e < (22 + (size_t)nc) * uT) { const size_t i = e - 22 * uT; at = (kColCount + i % nc) * a.tpad + i / nc; }
+        else {
+            const size_t i = e - (22 + (size_t)nc) * uT;
+            at = (size_t)kRowHead * a.tpad + i / a.nbvec * a.nb_pad + i % a.nbvec;
+        }
+        double s = 0.0;
+        for (int c = 0; c < ncopy; ++c) s += __ldcs(src + (size_t)c * a.row_sz + at);
+        dst[e] = s;
+    }
+}
 
 // Padded lattice: (n1+2) x (n2+2) x (n3+2), interior = the labels, border =
 // the wall code.  An interior voxel also gets the free-flight flag when its 26
@@ -576,6 +691,18 @@ int pack_lattice_padded(const uint8_t* labels, int n1, int n2, int n3, int bits,
         pad_pack_kernel<4><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(labels, n1, n2, n3, mirror, out, nbytes);
     else
         pad_pack_kernel<8><<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(labels, n1, n2, n3, mirror, out, nbytes);
+    return (int)cudaGetLastError();
+}
+
+int launch_gather_rows(const WalkArgs& a, double* out, size_t fields, void* stream) {
+    const size_t n = (size_t)a.timepoints * (kColCount + kNcMax + a.nbvec);
+    const unsigned gx = (unsigned)std::min<size_t>((n + 255) / 256, 1024);
+    for (int k = 0; k < a.naxons; k += 32768) {   // grid.y holds at most 65535 axons
+        WalkArgs b = a;
+        b.axons += k;
+        gather_rows_kernel<<<dim3(gx, (unsigned)std::min(32768, a.naxons - k)), 256, 0, (cudaStream_t)stream>>>(
+            b, out + (size_t)k * fields, fields);
+    }
     return (int)cudaGetLastError();
 }
 
