@@ -270,9 +270,9 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                 }
             }
             const int ai0 = (active && !resume) ? label_at<BITS>(lat, lin) : 0;
-            SplitWalker wk{lin, (active && !resume) ? cell_at<BITS>(lat, lin) : 0u, f0, f1, f2, 0, 0, 0, f0, f1, f2,
+            SplitWalker wk{lin, (active && !resume) ? cell_at<BITS>(lat, lin) : 0u, f0, f1, f2, 0.0f, 0.0f, 0.0f, f0, f1, f2,
                         ai0, t_step[ai0], t_k[ai0], 0.0f};
-            const SplitGeom geo{lat, s0, s1, a.nite, (bool)a.flight, (bool)a.same_cross, mirror};
+            const SplitGeom geo{lat, s0, s1, floor_bias(s0, s1), a.nite, (bool)a.flight, (bool)a.same_cross, mirror};
             auto nsize = [&](int axis) { return axis == 0 ? a.n1 : (axis == 1 ? a.n2 : a.n3); };
             DomainStream perm;
             perm.init(a.seed, (uint64_t)w, kDomPerm);
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                     wk.lin = c[0 * nw]; wk.cell = c[1 * nw];
                     wk.o0 = __uint_as_float(c[2 * nw]); wk.o1 = __uint_as_float(c[3 * nw]);
                     wk.o2 = __uint_as_float(c[4 * nw]);
-                    wk.D0 = (int)c[5 * nw]; wk.D1 = (int)c[6 * nw]; wk.D2 = (int)c[7 * nw];
+                    wk.D0 = __uint_as_float(c[5 * nw]); wk.D1 = __uint_as_float(c[6 * nw]); wk.D2 = __uint_as_float(c[7 * nw]);
                     wk.Fm0 = __uint_as_float(c[8 * nw]); wk.Fm1 = __uint_as_float(c[9 * nw]);
                     wk.Fm2 = __uint_as_float(c[10 * nw]);
                     wk.ai = (int)c[11 * nw];
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                         c[0 * nw] = wk.lin; c[1 * nw] = wk.cell;
                         c[2 * nw] = __float_as_uint(wk.o0); c[3 * nw] = __float_as_uint(wk.o1);
                         c[4 * nw] = __float_as_uint(wk.o2);
-                        c[5 * nw] = (uint32_t)wk.D0; c[6 * nw] = (uint32_t)wk.D1; c[7 * nw] = (uint32_t)wk.D2;
+                        c[5 * nw] = __float_as_uint(wk.D0); c[6 * nw] = __float_as_uint(wk.D1); c[7 * nw] = __float_as_uint(wk.D2);
                         c[8 * nw] = __float_as_uint(wk.Fm0); c[9 * nw] = __float_as_uint(wk.Fm1);
                         c[10 * nw] = __float_as_uint(wk.Fm2);
                         c[11 * nw] = (uint32_t)wk.ai;
@@ -378,11 +378,11 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                     split_step<NC, BITS, 0>(wk, v0, v1, v2, geo, t_step, t_k, t_pij, t_ratio, perm, nsize, h);
                 }
                 const float o0 = wk.o0, o1 = wk.o1, o2 = wk.o2;
-                const int D0 = wk.D0, D1 = wk.D1, D2 = wk.D2;
+                const float D0 = wk.D0, D1 = wk.D1, D2 = wk.D2;
                 const float Fm0 = wk.Fm0, Fm1 = wk.Fm1, Fm2 = wk.Fm2;
-                p0 += (float)D0 + (o0 - Fm0);
-                p1 += (float)D1 + (o1 - Fm1);
-                p2 += (float)D2 + (o2 - Fm2);
+                p0 += D0 + (o0 - Fm0);
+                p1 += D1 + (o1 - Fm1);
+                p2 += D2 + (o2 - Fm2);
                 if (p1st) { B0 += h.T0; B1 += h.T1; B2 += h.T2; }
                 const bool event = (i + 1 == next_bin);
                 if (event || (i & 31) == 31) {
@@ -420,9 +420,9 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                                 xb[nw] = (float)x1;
                                 xb[2 * nw] = (float)x2;
                             }
-                            const float xe0 = ((float)D0 + (o0 - Fm0)) * a.res,
-                                        xe1 = ((float)D1 + (o1 - Fm1)) * a.res,
-                                        xe2 = ((float)D2 + (o2 - Fm2)) * a.res;
+                            const float xe0 = (D0 + (o0 - Fm0)) * a.res,
+                                        xe1 = (D1 + (o1 - Fm1)) * a.res,
+                                        xe2 = (D2 + (o2 - Fm2)) * a.res;
                             const float tb = (float)(i + 1);
 #pragma unroll
                             for (int j = 0; j < NW; ++j) {
@@ -435,8 +435,8 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                     } else {
                         // time rescaling: at the end of bin b (time t = (b + 1) bin_steps dt)
                         // sum_j a_jw t (g_j,b - g_j,b+1) . x(t), g_j,nbins = 0
-                        const float xe0 = ((float)D0 + (o0 - Fm0)) * a.res, xe1 = ((float)D1 + (o1 - Fm1)) * a.res,
-                                    xe2 = ((float)D2 + (o2 - Fm2)) * a.res;
+                        const float xe0 = (D0 + (o0 - Fm0)) * a.res, xe1 = (D1 + (o1 - Fm1)) * a.res,
+                                    xe2 = (D2 + (o2 - Fm2)) * a.res;
                         const float tb = (float)(i + 1);   // steps (the waveform table carries dt)
 #pragma unroll
                         for (int j = 0; j < NW; ++j) {

@@ -251,7 +251,7 @@ __device__ __forceinline__ void park_walker(volatile uint32_t* p, const SplitWal
                                             float q0, float q1, float q2, float q3) {
     p[0] = w.lin; p[1] = w.cell;
     p[2] = __float_as_uint(w.o0); p[3] = __float_as_uint(w.o1); p[4] = __float_as_uint(w.o2);
-    p[5] = (uint32_t)w.D0; p[6] = (uint32_t)w.D1; p[7] = (uint32_t)w.D2;
+    p[5] = __float_as_uint(w.D0); p[6] = __float_as_uint(w.D1); p[7] = __float_as_uint(w.D2);
     p[8] = __float_as_uint(w.Fm0); p[9] = __float_as_uint(w.Fm1); p[10] = __float_as_uint(w.Fm2);
     p[11] = (uint32_t)w.ai; p[12] = __float_as_uint(w.cur_step); p[13] = __float_as_uint(w.cur_k);
     p[14] = __float_as_uint(w.w32);
@@ -262,7 +262,7 @@ __device__ __forceinline__ void unpark_walker(const volatile uint32_t* p, SplitW
                                               float& q0, float& q1, float& q2, float& q3) {
     w.lin = p[0]; w.cell = p[1];
     w.o0 = __uint_as_float(p[2]); w.o1 = __uint_as_float(p[3]); w.o2 = __uint_as_float(p[4]);
-    w.D0 = (int)p[5]; w.D1 = (int)p[6]; w.D2 = (int)p[7];
+    w.D0 = __uint_as_float(p[5]); w.D1 = __uint_as_float(p[6]); w.D2 = __uint_as_float(p[7]);
     w.Fm0 = __uint_as_float(p[8]); w.Fm1 = __uint_as_float(p[9]); w.Fm2 = __uint_as_float(p[10]);
     w.ai = (int)p[11]; w.cur_step = __uint_as_float(p[12]); w.cur_k = __uint_as_float(p[13]);
     w.w32 = __uint_as_float(p[14]);
@@ -377,9 +377,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
         }
         const int ai0 = active ? label_at<BITS>(lat, lin) : 0;
         // displacement = D + (offset - Fm) per axis
-        SplitWalker wk{lin, active ? cell_at<BITS>(lat, lin) : 0u, f0, f1, f2, 0, 0, 0, f0, f1, f2, ai0,
+        SplitWalker wk{lin, active ? cell_at<BITS>(lat, lin) : 0u, f0, f1, f2, 0.0f, 0.0f, 0.0f, f0, f1, f2, ai0,
                         t_step[ai0], t_k[ai0], 0.0f};
-        const SplitGeom geo{lat, s0, s1, a.nite, flight, same_certain, mirror};
+        const SplitGeom geo{lat, s0, s1, floor_bias(s0, s1), a.nite, flight, same_certain, mirror};
         auto nsize = [&](int axis) { return axis == 0 ? AXF(n1) : (axis == 1 ? AXF(n2) : AXF(n3)); };
         NoHooks hooks;
         DomainStream perm;
@@ -435,15 +435,15 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
             }
             // in-voxel offsets of the current position
             const float o0 = wk.o0, o1 = wk.o1, o2 = wk.o2;
-            const int D0 = wk.D0, D1 = wk.D1, D2 = wk.D2;
+            const float D0 = wk.D0, D1 = wk.D1, D2 = wk.D2;
             const float Fm0 = wk.Fm0, Fm1 = wk.Fm1, Fm2 = wk.Fm2;
 
             if (sums) {
                 // displacement sums (voxels): PGSE, prefix sums read at the
                 // lobe edges; waveforms, one sum per time bin
-                p0 += (float)D0 + (o0 - Fm0);
-                p1 += (float)D1 + (o1 - Fm1);
-                p2 += (float)D2 + (o2 - Fm2);
+                p0 += D0 + (o0 - Fm0);
+                p1 += D1 + (o1 - Fm1);
+                p2 += D2 + (o2 - Fm2);
                 const bool event = (i + 1 == next_ev);
                 if (event || (i & 31) == 31) {
                     P0 += (double)p0; P1 += (double)p1; P2 += (double)p2;
@@ -476,9 +476,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                 wk.w32 = 0.0f;
                 const float s0 = active ? expf(-(float)w64) : 0.0f;
                 const float res = AXF(res);
-                const float dx = ((float)D0 + (o0 - Fm0)) * res;
-                const float dy = ((float)D1 + (o1 - Fm1)) * res;
-                const float dz = ((float)D2 + (o2 - Fm2)) * res;
+                const float dx = (D0 + (o0 - Fm0)) * res;
+                const float dy = (D1 + (o1 - Fm1)) * res;
+                const float dz = (D2 + (o2 - Fm2)) * res;
                 float* st = s_stage[threadIdx.x >> 5] + 4;
                 unsigned* msk = s_mask[threadIdx.x >> 5];
                 float* mine = st + r * kStageRow + lane;

@@ -19,12 +19,23 @@
 
 namespace rms {
 
+// Floor of x in (-1, 2) on the FP32 pipe: x + 1.5 2^23, rounded down, has floor(x)
+// in its low bits and, less 1.5 2^23, as a float (both exact).  FRND and F2I do
+// the same on a pipe of a quarter to an eighth of the rate, which the record
+// sums' FP64 conversions also need.
+constexpr float kFloor = 12582912.0f;
+constexpr unsigned kFloorBits = 0x4B400000u;
+__device__ __forceinline__ unsigned floor_bias(int s0, int s1) { return kFloorBits * (unsigned)(s0 + s1 + 1); }
+
 // A walker between steps.
 struct SplitWalker {
     unsigned lin;            // voxel: linear index into the padded lattice
     unsigned cell;           // its lattice cell (label + free-flight flag)
     float o0, o1, o2;        // in-voxel offset along each axis, 0..1 (1: on the upper face)
-    int D0, D1, D2;          // integer part of the displacement: voxel - origin image
+    // integer part of the displacement, voxel - origin image, as floats: exact
+    // to 2^24 voxels, over 300 standard deviations of the longest walk (2^31
+    // steps shorter than a voxel), and read as floats every step
+    float D0, D1, D2;
     float Fm0, Fm1, Fm2;     // fractional part of the origin image (mirrored at walls)
     int ai;                  // compartment (label)
     float cur_step, cur_k;   // step length (voxels), T2 exponent per voxel of path
@@ -36,6 +47,7 @@ struct SplitWalker {
 struct SplitGeom {
     const uint8_t* lat;
     int s0, s1;              // padded strides of axes 0 and 1 (axis 2: 1)
+    unsigned bias;           // kFloorBits (s0 + s1 + 1): see kFloor
     int nite;
     bool flight;             // straight moves allowed (same-label faces always crossed, nite >= 4)
     bool same_certain;       // same-label faces are crossed without a draw
@@ -84,31 +96,34 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
         float x0 = fmaf(s.cur_step, v0, s.o0);
         float x1 = fmaf(s.cur_step, v1, s.o1);
         float x2 = fmaf(s.cur_step, v2, s.o2);
-        float k0 = floorf(x0), k1 = floorf(x1), k2 = floorf(x2);
-        int ik0 = (int)k0, ik1 = (int)k1, ik2 = (int)k2;
-        unsigned lj = s.lin + (unsigned)(ik0 * s0 + ik1 * s1 + ik2);
+        const float r0 = __fadd_rd(x0, kFloor), r1 = __fadd_rd(x1, kFloor), r2 = __fadd_rd(x2, kFloor);
+        float k0 = r0 - kFloor, k1 = r1 - kFloor, k2 = r2 - kFloor;
+        // lin + k0 s0 + k1 s1 + k2, the floors' common high bits taken off by the bias
+        unsigned lj = (s.lin - g.bias) + __float_as_uint(r0) * (unsigned)s0 + __float_as_uint(r1) * (unsigned)s1 +
+                      __float_as_uint(r2);
         unsigned cj = cell_at<BITS>(lat, lj);
         if ((cj & label_mask<BITS>()) == (unsigned)kWall) {
+            int ik0 = (int)k0, ik1 = (int)k1, ik2 = (int)k2;
             // out through one or more mirror walls: reflect on each axis whose
             // face neighbour is a wall (x -> -x below the voxel, 2 - x above)
             if (ik0 != 0 && label_at<BITS>(lat, s.lin + (unsigned)(ik0 * s0)) == kWall) {
                 const bool hi = ik0 > 0;
                 const int nh = nsize(0), gw = hi ? nh - 1 : 0;
-                int I = gw - s.D0; mirror_origin(I, s.Fm0, hi, nh); s.D0 = gw - I;
+                int I = gw - (int)s.D0; mirror_origin(I, s.Fm0, hi, nh); s.D0 = (float)(gw - I);
                 x0 = hi ? 2.0f - x0 : -x0; k0 = 0.0f; ik0 = 0;
                 h.reflect(0);
             }
             if (ik1 != 0 && label_at<BITS>(lat, s.lin + (unsigned)(ik1 * s1)) == kWall) {
                 const bool hi = ik1 > 0;
                 const int nh = nsize(1), gw = hi ? nh - 1 : 0;
-                int I = gw - s.D1; mirror_origin(I, s.Fm1, hi, nh); s.D1 = gw - I;
+                int I = gw - (int)s.D1; mirror_origin(I, s.Fm1, hi, nh); s.D1 = (float)(gw - I);
                 x1 = hi ? 2.0f - x1 : -x1; k1 = 0.0f; ik1 = 0;
                 h.reflect(1);
             }
             if (ik2 != 0 && label_at<BITS>(lat, s.lin + (unsigned)ik2) == kWall) {
                 const bool hi = ik2 > 0;
                 const int nh = nsize(2), gw = hi ? nh - 1 : 0;
-                int I = gw - s.D2; mirror_origin(I, s.Fm2, hi, nh); s.D2 = gw - I;
+                int I = gw - (int)s.D2; mirror_origin(I, s.Fm2, hi, nh); s.D2 = (float)(gw - I);
                 x2 = hi ? 2.0f - x2 : -x2; k2 = 0.0f; ik2 = 0;
                 h.reflect(2);
             }
@@ -117,7 +132,7 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
         }
         s.lin = lj;
         s.cell = cj;
-        s.D0 += ik0; s.D1 += ik1; s.D2 += ik2;
+        s.D0 += k0; s.D1 += k1; s.D2 += k2;
         s.w32 = fmaf(s.cur_step, s.cur_k, s.w32);
         h.path(s.ai, s.cur_step);
         s.o0 = x0 - k0; s.o1 = x1 - k1; s.o2 = x2 - k2;
@@ -168,9 +183,9 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
                 if (g.mirror) {
                     // mirror wall: reflect, and mirror the origin image
                     const int gw = hi ? nh - 1 : 0;
-                    if (hit == 0) { int I = gw - s.D0; mirror_origin(I, s.Fm0, hi, nh); s.D0 = gw - I; }
-                    else if (hit == 1) { int I = gw - s.D1; mirror_origin(I, s.Fm1, hi, nh); s.D1 = gw - I; }
-                    else { int I = gw - s.D2; mirror_origin(I, s.Fm2, hi, nh); s.D2 = gw - I; }
+                    if (hit == 0) { int I = gw - (int)s.D0; mirror_origin(I, s.Fm0, hi, nh); s.D0 = (float)(gw - I); }
+                    else if (hit == 1) { int I = gw - (int)s.D1; mirror_origin(I, s.Fm1, hi, nh); s.D1 = (float)(gw - I); }
+                    else { int I = gw - (int)s.D2; mirror_origin(I, s.Fm2, hi, nh); s.D2 = (float)(gw - I); }
                     aj = -1;   // reflect below
                 } else {
                     // periodic: the neighbour is on the far side; the
@@ -202,7 +217,7 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
                 s.ai = aj;
             }
             s.lin = lj;
-            const int du = ((up >> hit) & 1u) ? 1 : -1;
+            const float du = ((up >> hit) & 1u) ? 1.0f : -1.0f;
             if (hit == 0) s.D0 += du; else if (hit == 1) s.D1 += du; else s.D2 += du;
         } else {
             up ^= 1u << hit;
