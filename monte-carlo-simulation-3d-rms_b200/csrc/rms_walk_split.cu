@@ -234,12 +234,19 @@ __device__ __noinline__ void add_signals(const float* st, const double* __restri
                     bz = in ? (float)__ldg(bvec + jb * 3 + 2) : 0.0f;
         for (int r = 0; r < nrec; ++r) {
             const float q = in ? (float)__ldg(qtab + (size_t)r * nb + jb) : 0.0f;
+            const float* v = st + r * kStageRow;
+            auto cosine = [&](float dx, float dy, float dz, float s0) {
+                const float qx = q * (dx * bx + dy * by + dz * bz);
+                return (double)(s0 * cosf(qx));
+            };
             double s = 0.0;
-#pragma unroll 4
-            for (int w = 0; w < nw; ++w) {
-                const float* v = st + r * kStageRow + w;
-                const float qx = q * (v[0] * bx + v[32] * by + v[64] * bz);
-                s += (double)(v[96] * cosf(qx));
+#pragma unroll 1
+            for (int w = 0; w < nw; w += 4) {
+                // past the tile's walkers the weights are zero
+                const float4 X = *reinterpret_cast<const float4*>(v + w), Y = *reinterpret_cast<const float4*>(v + 32 + w),
+                             Z = *reinterpret_cast<const float4*>(v + 64 + w), S = *reinterpret_cast<const float4*>(v + 96 + w);
+                s += (cosine(X.x, Y.x, Z.x, S.x) + cosine(X.y, Y.y, Z.y, S.y)) +
+                     (cosine(X.z, Y.z, Z.z, S.z) + cosine(X.w, Y.w, Z.w, S.w));
             }
             if (in) add_out<ONE>(dst + (size_t)r * stride + jb, s);
         }
