@@ -79,6 +79,7 @@ struct WalkArgs {
     // signals into out_sig[axon][ngrad_pad]
     const AxonDesc* axons;
     int naxons;
+    int tile_w;                 // table form: walkers of a tile, one warp's, 1..32
     int64_t ntiles;
     double* rows;
     int tpad, nb_pad;

@@ -155,8 +155,8 @@ constexpr int kStageOnes = -4;          // before the first record, four ones
 // flush when a warp moves on to another axon.
 template <int KR, bool ONE>
 __device__ __noinline__ void add_moments(const float* st, const unsigned* msk, double* dst, int stride, int nrec,
-                                         unsigned act, int nc, int lane) {
-    constexpr int NW = 4 * KR;   // walkers per lane
+                                         unsigned act, int nc, int nw, int lane) {
+    constexpr int NW = 4 * KR;   // walkers per lane, of the tile's nw (the rest weigh nothing)
     const int r = lane & (KR - 1), g = (lane / KR) & 3, half = lane / (4 * KR);
     __syncwarp();
     double q0 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0, q4 = 0.0, q5 = 0.0;
@@ -165,7 +165,7 @@ __device__ __noinline__ void add_moments(const float* st, const unsigned* msk, d
     const float* mp = g == 0 ? st + kStageOnes : row_st + (g - 1) * 32;
     const int minc = g == 0 ? 0 : 4;
 #pragma unroll 1
-    for (int k = 0; k < NW; k += 4, mp += minc) {
+    for (int k = 0; k < min(NW, nw - half * NW); k += 4, mp += minc) {
         const float4 X = *reinterpret_cast<const float4*>(row_st + k), Y = *reinterpret_cast<const float4*>(row_st + 32 + k),
                      Z = *reinterpret_cast<const float4*>(row_st + 64 + k),
                      S = *reinterpret_cast<const float4*>(row_st + 96 + k), M = *reinterpret_cast<const float4*>(mp);
@@ -359,8 +359,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
         const float* t_ratio = tab + 2 * NCMAX + NCMAX * NCMAX;
         const uint32_t key0 = (uint32_t)seed, key1 = (uint32_t)(seed >> 32);
 
-        const int64_t w = AXF(walker_begin) + (tile - (ONE ? 0 : AXF(tile_begin))) * 32 + lane;
-        bool active = w < AXF(walker_end);
+        // (the walkers past a narrow tile are the next tile's)
+        const int tile_w = ONE ? 32 : a.tile_w;
+        const int64_t w = AXF(walker_begin) + (tile - (ONE ? 0 : AXF(tile_begin))) * tile_w + lane;
+        bool active = w < AXF(walker_end) && lane < tile_w;
         const uint32_t wlo = (uint32_t)w, whi = (uint32_t)((uint64_t)w >> 32);
 
         // initial position: uniform in the labelled voxels (rejection sampling)
@@ -504,12 +506,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                     double* set = ONE ? a.slots + (size_t)warp_global * a.timepoints * a.nvals
                                       : a.rows + AXF(row_off) + (size_t)(warp_global % AXF(ncopy)) * a.row_sz;
                     add_moments<KR, ONE>(st, msk, ONE ? set + (size_t)rec0 * a.nvals : set + rec0,
-                                         ONE ? a.nvals : a.tpad, rec - rec0, act, AXF(nc), lane);
+                                         ONE ? a.nvals : a.tpad, rec - rec0, act, AXF(nc), tile_w, lane);
                     if (!sums && a.nbvec > 0)
                         add_signals<ONE>(st, a.qtab + (size_t)rec0 * a.nbvec, a.bvec, a.nbvec,
                                          ONE ? set + (size_t)rec0 * a.nvals + kRowHead
                                              : set + (size_t)kRowHead * a.tpad + (size_t)rec0 * a.nb_pad,
-                                         ONE ? a.nvals : a.nb_pad, rec - rec0, 32, lane);
+                                         ONE ? a.nvals : a.nb_pad, rec - rec0, tile_w, lane);
                     __syncwarp();
                     unpark_walker(park, wk, perm, q0, q1, q2, q3);
                 }

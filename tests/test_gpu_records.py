@@ -68,3 +68,19 @@ def test_every_other_record_of_one_walk(nc):
     assert np.array_equal(coarse["npar_count"], fine["npar_count"][::2])
     for k in ("sig0", "dx2", "dx4"):
         np.testing.assert_allclose(coarse[k], fine[k][::2], rtol=1e-12, atol=1e-18)
+
+
+@pytest.mark.parametrize("npar", [1, 2, 1776, 1777, 3553, 20000])
+def test_narrow_tiles_walk_the_same_walkers(npar):
+    """Small launches walk fewer than 32 walkers a warp.  A launch's walkers are
+    those of its shards, whose tiles have other widths and edges; the sums differ
+    by their order alone."""
+    sim = make(9, 20, npar, 3, T2=(80.0, 40.0))[0]
+    whole = sim.run(seed=2, precision="split").outputs()
+    parts = [make(9, 20, npar, 3, T2=(80.0, 40.0))[0].run(seed=2, precision="split", shard=(i, 3)).outputs()
+             for i in range(3)]
+    assert np.array_equal(sum(p["npar_count"] for p in parts), whole["npar_count"])
+    assert np.array_equal(whole["npar_count"].sum(axis=1), np.full(9, float(npar)))
+    for k in ("sig0", "dx2", "dx4", "sigre"):
+        scale = np.abs(whole[k]).max()
+        assert np.abs(sum(p[k] for p in parts) - whole[k]).max() <= 1e-12 * scale * max(1, npar ** 0.5), k
