@@ -54,8 +54,15 @@ RMS_HD U4 philox4x32_10(U4 c, uint32_t k0, uint32_t k1) {
 }
 
 RMS_HD double u53_to_double(uint32_t lo, uint32_t hi) {
+#if defined(__CUDA_ARCH__)
+    // the same value from the bits: 1 + m 2^-52 (m the 52 top bits) minus
+    // (1 - 2^-53), exact (Sterbenz)
+    return __dsub_rn(__hiloint2double((int)(0x3ff00000u | (hi >> 12)), (int)((hi << 20) | (lo >> 12))),
+                     1.0 - 0x1p-53);
+#else
     const uint64_t m = ((((uint64_t)hi) << 32) | lo) >> 12;
     return (double)(2 * m + 1) * 0x1p-53;
+#endif
 }
 
 RMS_HD float u32_to_float(uint32_t x) {
@@ -89,6 +96,17 @@ struct DoubleStream {
         spare = u53_to_double(r.z, r.w);
         has_spare = true;
         return u53_to_double(r.x, r.y);
+    }
+    // The next two doubles.  One block whether or not a spare is held (the spare
+    // moves on by two), so lanes whose other draws left them out of step still
+    // generate it together.
+    RMS_HD void next2(double& a, double& b) {
+        const U4 r = philox4x32_10(U4{(uint32_t)block, (uint32_t)(block >> 32), w0, w1}, k0, k1);
+        ++block;
+        const double d0 = u53_to_double(r.x, r.y), d1 = u53_to_double(r.z, r.w);
+        a = has_spare ? spare : d0;
+        b = has_spare ? d0 : d1;
+        spare = d1;
     }
 };
 

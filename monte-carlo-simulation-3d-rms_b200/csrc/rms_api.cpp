@@ -509,9 +509,34 @@ int split_row_sets(int64_t warps, size_t row_sz) {
 //   2e4           32: 2.46  16: 2.23  12: 2.12   8: 2.28
 //   5e4           32: 2.89  28: 2.80  24: 2.73  16: 2.77
 //   1e5           32: 3.48  28: 3.95  16: 4.68
-int split_tile_width(int64_t nwalk, int sms) {
+int tile_width(int64_t nwalk, int sms) {
     const int64_t warps = (int64_t)3 * 4 * sms;
     return (int)std::min<int64_t>(32, std::max<int64_t>(1, (nwalk + warps - 1) / warps));
+}
+
+// The COMPAT walk's form (4, 5 or 6 resident blocks of four warps per SM) for
+// ntiles tiles: the one whose rounds end first.  A round of 5 blocks takes 1.16
+// times a round of 4, of 6 blocks 1.44 times (1e6 walkers x 500 steps: 21.3 /
+// 19.7 / 20.5 ms); 1e5 walkers (3125 tiles) x 2000 steps take 26.2 ms in two
+// rounds of 4 blocks and 20.5 in one of 6.
+// More than 4 only while the warps' rows (row_bytes each) stay under 4 GB.
+int compat_form(const rms_sim* s, bool trace, int sms, int64_t ntiles, int64_t row_bytes, int& per_sm) {
+    int best = 4;
+    double least = 0.0;
+    per_sm = -1;
+    for (int b = 4; b <= (trace ? 4 : 6); ++b) {
+        const int n = walk_compat_blocks_per_sm(s->nc, trace, s->mode == RMS_MODE_PGSE, b);
+        if (n < 1 || (n < b && b > 4)) continue;
+        const int64_t slots = (int64_t)sms * n * (kCompatBlock / 32);
+        if (b > 4 && std::min(slots, ntiles) * row_bytes > (int64_t)4 << 30) continue;
+        const double t = (double)((ntiles + slots - 1) / slots) * (b == 4 ? 1.0 : (b == 5 ? 1.16 : 1.44));
+        if (per_sm < 0 || t < least) {
+            best = b;
+            least = t;
+            per_sm = n;
+        }
+    }
+    return best;
 }
 
 // Settings every simulation of one split launch must share (the signal
@@ -574,11 +599,21 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
     // launch shape: persistent grid
     int dev_sms = 0;
     RMS_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device));
-    int block = kCompatBlock, per_sm, variant = 0, lattice_bits = 8;
+    int block = kCompatBlock, per_sm = -1, variant = 0, lattice_bits = 8;
     int nc_max = 0;
     for (LaunchJob& j : jobs) nc_max = std::max(nc_max, j.s->nc);
+    int64_t nwalk = 0;
+    for (const LaunchJob& j : jobs) nwalk += j.w1 - j.w0;
+    const int T = s->timepoints;
+    const int nb = s->nbvec();
+    const int nvals = (s->mode == RMS_MODE_NARROW) ? kRowHead + ((nb + 31) / 32) * 32 : kRowHead;
+    int tile_w = tile_width(nwalk, dev_sms);
     if (prec == RMS_PREC_COMPAT) {
-        per_sm = walk_compat_blocks_per_sm(s->nc, trace_n > 0);
+        // every warp has its own rows: narrow tiles only as far as these stay under 1 GB
+        const int64_t row_bytes = (int64_t)T * nvals * (int64_t)sizeof(double);
+        const int64_t most = ((int64_t)1 << 30) / row_bytes;
+        tile_w = (int)std::min<int64_t>(32, std::max<int64_t>(tile_w, nwalk / std::max<int64_t>(most, 1) + 1));
+        variant = compat_form(s, trace_n > 0, dev_sms, (nwalk + tile_w - 1) / tile_w, row_bytes, per_sm);
     } else {
         lattice_bits = split_lattice_bits(nc_max);
         variant = (o && o->variant > 0) ? o->variant - 1 : kSplitVariantDefault;
@@ -588,9 +623,6 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
         per_sm = walk_split_blocks_per_sm(nc_max, lattice_bits, variant);
     }
     if (per_sm <= 0) return set_error(RMS_ERR_CUDA, "occupancy query failed (kernel image missing for this GPU?)");
-    int64_t nwalk = 0;
-    for (const LaunchJob& j : jobs) nwalk += j.w1 - j.w0;
-    const int tile_w = prec == RMS_PREC_SPLIT ? split_tile_width(nwalk, dev_sms) : 32;
     std::vector<int64_t> tile_begin(naxons + 1, 0);
     for (int k = 0; k < naxons; ++k)
         tile_begin[k + 1] = tile_begin[k] + (jobs[k].w1 - jobs[k].w0 + tile_w - 1) / tile_w;
@@ -600,16 +632,13 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
     const int grid = (int)std::max<int64_t>(grid64, 1);
     const int nthr = grid * block;
     const int nwarps = nthr / 32;
-    const int T = s->timepoints;
-    const int nb = s->nbvec();
-    const int nvals = (s->mode == RMS_MODE_NARROW) ? kRowHead + ((nb + 31) / 32) * 32 : kRowHead;
     const bool wavemode = s->mode == RMS_MODE_WAVEFORM;
     const bool has_sig = s->mode != RMS_MODE_NARROW;
     // signal row: PGSE, one value per gradient; waveforms, (cos, sin) per waveform
     const int ngrad = wavemode ? 2 * s->nwave : s->ngrad();
     const int ngrad_pad = std::max(32, ((ngrad + 31) / 32) * 32);
 
-    const int nseg = nwarps;   // COMPAT: one accumulator row set per warp
+    const int nseg = (int)std::min<int64_t>(nwarps, ntiles);   // COMPAT: the warps that walk, each with its own rows
     // The SPLIT walk runs in the table form (axon fields and seeds from device
     // memory, tiles from a queue, records added into a few row sets per axon
     // with FP64 atomics): for one axon too, where it is 1.3x faster than the
@@ -746,15 +775,12 @@ int enqueue_launch(LaunchPlan& p, rms_sim* s, bool events) {
     const WalkArgs& a = p.a;
     if (p.prec == RMS_PREC_SPLIT)
         RMS_CUDA(cudaMemcpyAsync(d->axons.p, d->h_axons.p, sizeof(AxonDesc) * p.naxons, cudaMemcpyHostToDevice, st));
+    // (a COMPAT warp's first tile stores its rows: they need no clearing)
     if (p.multi) RMS_CUDA(cudaMemsetAsync(d->rows.p, 0, p.nsets * sizeof(double), st));
-    else RMS_CUDA(cudaMemsetAsync(d->slots.p, 0, (size_t)p.nseg * p.row * sizeof(double), st));
     RMS_CUDA(cudaMemsetAsync(d->err.p, 0, 16, st));
-    if (p.has_sig) {
-        if (p.multi) RMS_CUDA(cudaMemsetAsync(d->out_sig.p, 0, p.nsig * sizeof(double), st));
-        else RMS_CUDA(cudaMemsetAsync(d->sig_slots.p, 0, (size_t)p.nseg * p.ngrad_pad * sizeof(double), st));
-    }
+    if (p.multi && p.has_sig) RMS_CUDA(cudaMemsetAsync(d->out_sig.p, 0, p.nsig * sizeof(double), st));
     if (events) RMS_CUDA(cudaEventRecord(d->e0, st));
-    int e = (p.prec == RMS_PREC_COMPAT) ? launch_walk_compat(a, p.grid, p.block, p.trace_n > 0, st)
+    int e = (p.prec == RMS_PREC_COMPAT) ? launch_walk_compat(a, p.grid, p.block, p.variant, p.trace_n > 0, st)
                                         : launch_walk_split(a, p.bits, p.variant, p.grid, st);
     if (e) return cuda_fail((cudaError_t)e, "walk kernel launch");
     if (events) RMS_CUDA(cudaEventRecord(d->e1, st));

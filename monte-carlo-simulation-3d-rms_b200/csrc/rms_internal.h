@@ -79,7 +79,7 @@ struct WalkArgs {
     // signals into out_sig[axon][ngrad_pad]
     const AxonDesc* axons;
     int naxons;
-    int tile_w;                 // table form: walkers of a tile, one warp's, 1..32
+    int tile_w;                 // walkers of a tile, one warp's, 1..32 (the no-allocation form: 32)
     int64_t ntiles;
     double* rows;
     int tpad, nb_pad;
@@ -105,7 +105,7 @@ struct WalkArgs {
 
 // Launchers (rms_walk_*.cu, rms_reduce.cu).  All asynchronous on `stream`;
 // they return a cudaError_t value (0 = success).
-int launch_walk_compat(const WalkArgs& a, int grid, int block, bool trace, void* stream);
+int launch_walk_compat(const WalkArgs& a, int grid, int block, int minb, bool trace, void* stream);
 // Split walk over a.naxons axons (a.axons, a.ntiles, and a.rows/out_sig, or the
 // no-allocation form's per-warp a.slots); lattice_bits: packed lattice format.
 int launch_walk_split(const WalkArgs& a, int lattice_bits, int variant, int grid, void* stream);
@@ -126,7 +126,8 @@ int pack_lattice_padded(const uint8_t* labels, int n1, int n2, int n3, int bits,
                         void* stream);
 int launch_reduce_slots(const double* slots, int nslots, size_t row, double* out, void* stream);
 // Resident blocks per SM of the walk kernels (occupancy API); -1 on error.
-int walk_compat_blocks_per_sm(int nc, bool trace);
+// (minb: the COMPAT walk's form, built for 4, 5 or 6 resident blocks)
+int walk_compat_blocks_per_sm(int nc, bool trace, bool pgse, int minb);
 int walk_split_blocks_per_sm(int nc, int lattice_bits, int variant);
 const char* cuda_error_string(int code);
 

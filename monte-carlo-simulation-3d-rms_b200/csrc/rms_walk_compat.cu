@@ -23,7 +23,6 @@
 
 #include "philox.cuh"
 #include "rms_internal.h"
-#include "warp_reduce.cuh"
 
 namespace rms {
 namespace {
@@ -31,45 +30,150 @@ namespace {
 constexpr double kRefPi = 3.14159265;  // main.cu:34 (the reference's truncated pi)
 constexpr int kBlock = 128;
 
-template <int NCMAX>
-__device__ __forceinline__ void add_residence(double (&tc)[NCMAX], int c, double x) {
-#pragma unroll
-    for (int k = 0; k < NCMAX; ++k)
-        if (k == c) tc[k] = tc[k] + x;
-}
-
 __device__ __forceinline__ unsigned lin3(int i, int j, int k, int n2, int n3) {
     return ((unsigned)i * (unsigned)n2 + (unsigned)j) * (unsigned)n3 + (unsigned)k;
 }
 
-// Nearest face along the ray on one axis (main.cu:200-219).
-__device__ __forceinline__ void face(int axis, double v, double x, int g, double& tmin, int& hit) {
-    double tmp;
-    if (v > 0.0) {
-        tmp = (double)g + 1.0 - x;
-    } else if (v < 0.0) {
-        tmp = (double)g - x;
-    } else {
-        tmp = 2.0;
-    }
-    double tt;
-    if (fabs(tmp) > fabs(v)) {
-        tt = 2.0;
-    } else {
-        const double q = tmp / v;
-        tt = (0.0 < q) ? q : 0.0;  // std::max(0.0, q)
-    }
-    if (tt < tmin) { tmin = tt; hit = axis; }
+// Time to the face ahead on one axis, as the reference forms it (main.cu:200-219):
+// d = face - x, beyond a whole step 2, never negative.
+__device__ __forceinline__ double face_time(double d, double v) {
+    if (fabs(d) > fabs(v)) return 2.0;
+    const double q = d / v;
+    return (0.0 < q) ? q : 0.0;  // std::max(0.0, q)
 }
 
-template <int NCMAX, bool TRACE>
-__global__ void __launch_bounds__(kBlock) walk_compat_kernel(const WalkArgs a) {
-    __shared__ double s_step[NCMAX], s_t2[NCMAX], s_pij[NCMAX * NCMAX];
+// a / b rounded to nearest from y = 1 / b rounded to nearest: two residual
+// corrections of a * y.  The first leaves a quotient within an ulp, from which
+// the second is the correctly rounded one (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990, theorem 8.3) -- the division's own result, without forming the
+// reciprocal of the same b again for every a.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// Records in batches of kRec, as the split walk takes them
+// (rms_walk_split.cu): every lane stages its walker's displacement and T2
+// weight, then lane (r, g) adds six of record r's moments over the tile's
+// walkers; lane j of the signals holds one b-value.  One record at a time cost
+// a 32-value FP64 reduce-scatter (~270 instructions), and each b-value 10
+// shuffles and 5 adds after its cosine.
+constexpr int kRec = 8;
+// doubles of a staged record: x, y, z, s0 of 32 walkers, then 16 bytes that keep
+// the rows of a batch on different banks and hold the bits of the labels
+constexpr int kStageRow = 4 * 32 + 2;
+__device__ __forceinline__ unsigned* stage_masks(double* row) { return reinterpret_cast<unsigned*>(row + 4 * 32); }
+
+// A value into the warp's row: the warp's first tile stores, later ones add
+// (so the rows need no clearing).
+__device__ __forceinline__ void put(double* p, double x, bool first) { *p = first ? x : *p + x; }
+
+__device__ __noinline__ void add_moments(double* st, double* row, int nvals, int nrec, unsigned act,
+                                         int nw, bool first, int lane) {
+    const int r = lane & (kRec - 1), g = lane / kRec;
+    __syncwarp();
+    double q0 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0, q4 = 0.0, q5 = 0.0;
+    const double* v = st + r * kStageRow;
+#pragma unroll 2
+    for (int w = 0; w < nw; ++w) {
+        const double x = v[w], y = v[32 + w], z = v[64 + w], s0 = v[96 + w];
+        const double m = g == 1 ? x : (g == 2 ? y : z);
+        const double A = g == 0 ? s0 : s0 * m * m, Ax = A * x, Ay = A * y;
+        q0 += g == 2 ? s0 : Ax * x;
+        q1 += Ax * y;
+        q2 += Ax * z;
+        q3 += Ay * y;
+        q4 += Ay * z;
+        q5 += A * z * z;
+    }
+    if (r >= nrec) return;
+    row += (size_t)r * nvals;
+    // columns of the group's six products (-1: another group's)
+    const int c0 = g == 0 ? 1 : (g == 1 ? 7 : (g == 2 ? 0 : -1));
+    const int c1 = g == 0 ? 2 : (g == 1 ? 8 : (g == 2 ? 13 : 15));
+    const int c3 = g == 0 ? 4 : (g == 1 ? 10 : (g == 2 ? 17 : -1));
+    const int c4 = g == 0 ? 5 : (g == 1 ? 11 : (g == 2 ? 18 : 20));
+    if (c0 >= 0) put(row + c0, q0, first);
+    put(row + c1, q1, first);
+    put(row + c1 + 1, q2, first);
+    if (c3 >= 0) put(row + c3, q3, first);
+    put(row + c4, q4, first);
+    put(row + c4 + 1, q5, first);
+    const unsigned* msk = stage_masks(st + r * kStageRow);
+    const unsigned m0 = msk[0], m1 = msk[1], m2 = msk[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int c = 2 * g + k;
+        const int cnt = __popc(act & ((c & 1) ? m0 : ~m0) & ((c & 2) ? m1 : ~m1) & ((c & 4) ? m2 : ~m2));
+        put(row + kColCount + c, (double)cnt, first);
+    }
+}
+
+// narrow-pulse signals of a batch (main.cu:374-378)
+__device__ __noinline__ void add_signals(const double* st, const double* __restrict__ qtab,
+                                         const double* __restrict__ bvec, int nb, double* row, int nvals, int nrec,
+                                         int nw, bool first, int lane) {
+    __syncwarp();
+    for (int jb = lane; jb < nb; jb += 32) {
+        const double bx = __ldg(bvec + jb * 3), by = __ldg(bvec + jb * 3 + 1), bz = __ldg(bvec + jb * 3 + 2);
+        for (int r = 0; r < nrec; ++r) {
+            const double q = __ldg(qtab + (size_t)r * nb + jb);
+            const double* v = st + r * kStageRow;
+            double s = 0.0;
+#pragma unroll 2
+            for (int w = 0; w < nw; ++w) s += v[96 + w] * cos(q * (v[w] * bx + v[32 + w] * by + v[64 + w] * bz));
+            put(row + (size_t)r * nvals + jb, s, first);
+        }
+    }
+}
+
+// Final T2-weighted PGSE signal of the tile (main_PGSE.cu:348-357), lane j one
+// gradient: phase_j = |g| (g_hat . V) dt with the walkers' window sums V in vscr
+// ([pair * 3 + axis][thread], thread t0 + w).
+__device__ __noinline__ void add_pgse(const WalkArgs& a, int nthr, int t0, double s0, int nw, double* sig, bool first,
+                                      int lane) {
+    __syncwarp();
+    for (int base = 0; base < a.ngrad; base += 32) {
+        const int j = min(base + lane, a.ngrad - 1);
+        const double* g = a.grad + 6 * j;
+        const double* vv = a.vscr + (size_t)(a.gpair[j] * 3) * nthr + t0;
+        const double g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5];
+        double s = 0.0;
+        for (int w = 0; w < nw; ++w) {
+            const double phase = g2 * (vv[w] * g3 + vv[nthr + w] * g4 + vv[2 * (size_t)nthr + w] * g5) * a.dt;
+            s += __shfl_sync(0xffffffffu, s0, w) * cos(phase);
+        }
+        if (base + lane < a.ngrad) put(sig + j, s, first);
+    }
+}
+
+// What bounds it: FP64 issue (64 lanes per clock and SM) and, below a few warps
+// per scheduler, the latency of a step's FP64 chain.  So a step forms no
+// quotient it does not need: per axis the face ahead f (an integer kept as a
+// double), 1 / v once a step, and the time to a face as (f - x) / v only
+// approximately (2^-52) to choose the axis; the exact quotient is formed for the
+// axis that is hit, from the same reciprocal.  Where two faces, or a face and
+// the step's end, lie within 2^-46 of each other, the segment is decided by the
+// exact quotients of all three.  Every value that reaches the walker is the
+// reference's expression, rounded as written.
+//
+// MINB, resident blocks per SM: 4 (113 registers), 5 (96, 24 bytes spilled) or 6
+// (80, 156 bytes); the launch takes the one whose rounds of tiles end first
+// (compat_form in rms_api.cpp).
+template <int NCMAX, bool TRACE, bool PGSE, int MINB>
+__global__ void __launch_bounds__(kBlock, MINB) walk_compat_kernel(const __grid_constant__ WalkArgs a) {
+    __shared__ double s_step[NCMAX], s_rstep[NCMAX], s_t2[NCMAX], s_rt2[NCMAX], s_pij[NCMAX * NCMAX];
+    __shared__ double s_tc[NCMAX][kBlock];               // residence of the walker per compartment
+    __shared__ double s_stage[kBlock / 32][kRec * kStageRow];
     for (int i = threadIdx.x; i < NCMAX * NCMAX; i += blockDim.x) {
         s_pij[i] = (i < a.nc * a.nc) ? a.pij[i] : 0.0;
         if (i < NCMAX) {
             s_step[i] = (i < a.nc) ? a.step[i] : 0.0;
             s_t2[i] = (i < a.nc) ? a.t2[i] : 1.0;
+            s_rstep[i] = __drcp_rn(s_step[i]);
+            s_rt2[i] = __drcp_rn(s_t2[i]);
         }
     }
     __syncthreads();
@@ -79,157 +183,210 @@ __global__ void __launch_bounds__(kBlock) walk_compat_kernel(const WalkArgs a) {
     const int nthr = gridDim.x * blockDim.x;
     const int warp_global = gtid >> 5;
     const int nwarps = nthr >> 5;
-    const int64_t nwalk = a.walker_end - a.walker_begin;
-    const int64_t ntiles = (nwalk + 31) / 32;
-    const bool pgse = (a.mode == 1);
     const bool mirror = (a.boundary == 0);
     double* slot = a.slots + (size_t)warp_global * a.timepoints * a.nvals;
-    double* sig_slot = pgse ? a.sig_slots + (size_t)warp_global * a.ngrad_pad : nullptr;
+    double* st = s_stage[threadIdx.x >> 5];
+    const double n0 = (double)a.n1, n1 = (double)a.n2, n2 = (double)a.n3;
+    const int l0 = a.n2 * a.n3, l1 = a.n3;               // strides of the label lattice
+    constexpr double kNear = 1.0 + 0x1p-46;
 
-    for (int64_t tile = warp_global; tile < ntiles; tile += nwarps) {
-        const int64_t w = a.walker_begin + tile * 32 + lane;
-        bool active = w < a.walker_end;
+    for (int64_t tile = warp_global; tile < a.ntiles; tile += nwarps) {
+        const bool first = tile == warp_global;
+        const int64_t w = a.walker_begin + tile * a.tile_w + lane;
+        bool active = w < a.walker_end && lane < a.tile_w;
         DoubleStream rng;
         rng.init(a.seed, (uint64_t)w);
 
-        // initial position: rejection sampling in the box (main.cu:117-125)
+        // initial position: rejection sampling in the box (main.cu:117-132)
         double xi0 = 0.0, xi1 = 0.0, xi2 = 0.0;
-        int g0 = 0, g1 = 0, g2 = 0;
+        int lin = 0;
+        double g0 = 0.0, g1 = 0.0, g2 = 0.0;             // the voxel
+        int ai = 0;
         if (active) {
             long long tries = 0;
             for (;;) {
-                xi0 = rng.next() * (double)a.n1;
-                xi1 = rng.next() * (double)a.n2;
-                xi2 = rng.next() * (double)a.n3;
-                g0 = (int)floor(xi0); g1 = (int)floor(xi1); g2 = (int)floor(xi2);
-                if (__ldg(a.labels + lin3(g0, g1, g2, a.n2, a.n3)) != 0) break;
+                xi0 = rng.next() * n0;
+                xi1 = rng.next() * n1;
+                xi2 = rng.next() * n2;
+                const int i0 = (int)floor(xi0), i1 = (int)floor(xi1), i2 = (int)floor(xi2);
+                lin = (int)lin3(i0, i1, i2, a.n2, a.n3);
+                ai = (int)__ldg(a.labels + lin);
+                g0 = (double)i0; g1 = (double)i1; g2 = (double)i2;
+                if (ai != 0) break;
                 if (++tries >= kInitTryCap) { atomicOr(a.err, kErrInitCap); active = false; break; }
             }
         }
-        // main.cu:129-132
         double xt0 = xi0, xt1 = xi1, xt2 = xi2;
-        g0 = (int)floor(xt0); g1 = (int)floor(xt1); g2 = (int)floor(xt2);
-        int ai = active ? (int)__ldg(a.labels + lin3(g0, g1, g2, a.n2, a.n3)) : 0;
-        if (TRACE && active && w < a.trace_n) a.tr_init[w] = (int32_t)lin3(g0, g1, g2, a.n2, a.n3);
+        if (TRACE && active && w < a.trace_n) a.tr_init[w] = lin;
 
-        double tc[NCMAX];
+        double tcur = 0.0;                               // residence in compartment ai (the others': s_tc)
 #pragma unroll
-        for (int k = 0; k < NCMAX; ++k) tc[k] = 0.0;
+        for (int k = 0; k < NCMAX; ++k) s_tc[k][threadIdx.x] = 0.0;
+        // the T2 weight (main.cu:335-337)
+        auto weight = [&]() {
+            double s = 0.0;
+            s_tc[ai][threadIdx.x] = tcur;
+#pragma unroll
+            for (int c = 0; c < NCMAX; ++c)
+                if (c < a.nc) {
+                    const double tc = s_tc[c][threadIdx.x], y = s_rt2[c];
+                    s = s + (y > 0.0 ? div_by(tc, s_t2[c], y) : tc / s_t2[c]);   // (T2 may be infinite)
+                }
+            return active ? exp(-1.0 * s) : 0.0;
+        };
 
         // PGSE: running displacement sum and the lobe-edge events
         double p0 = 0.0, p1 = 0.0, p2 = 0.0;
         int evi = 0;
-        int next_ev = (pgse && a.nevents > 0) ? a.ev_step[0] : -1;
-        if (pgse)
+        int next_ev = (PGSE && a.nevents > 0) ? a.ev_step[0] : -1;
+        if (PGSE)
             for (int k = 0; k < a.npairs * 3; ++k) a.vscr[(size_t)k * nthr + gtid] = 0.0;
 
         int next_rec = 0, rec = 0;   // the next recorded step and its record
         for (int i = 0; i < a.tn; ++i) {                            // main.cu:134
             if (active) {
                 double fstep = 1.0;
-                unsigned f0 = 0u, f1 = 0u;
+                unsigned wall0 = 0u, wall1 = 0u;
                 uint32_t ev = 0u;
                 int nev = 0;
                 // direction (main.cu:140-151)
-                double vr = rng.next();
+                double vr, vr2;
+                rng.next2(vr, vr2);
                 const double cos_t = 1.0 - 2.0 * vr;
                 const double sin_t = 2.0 * sqrt(vr * (1.0 - vr));
-                vr = rng.next();
-                double v0 = sin_t * cos(2.0 * kRefPi * vr);
-                double v1 = sin_t * sin(2.0 * kRefPi * vr);
+                double sn, cs;
+                sincos(2.0 * kRefPi * vr2, &sn, &cs);
+                double v0 = sin_t * cs;
+                double v1 = sin_t * sn;
                 double v2 = cos_t;
+                double y0 = __drcp_rn(v0), y1 = __drcp_rn(v1), y2 = __drcp_rn(v2);
+                // the face ahead on each axis (no component is zero: both uniforms are odd multiples of 2^-53)
+                unsigned ups = (v0 > 0.0 ? 1u : 0u) | (v1 > 0.0 ? 2u : 0u) | (v2 > 0.0 ? 4u : 0u);
+                double f0 = (ups & 1u) ? g0 + 1.0 : g0, f1 = (ups & 2u) ? g1 + 1.0 : g1, f2 = (ups & 4u) ? g2 + 1.0 : g2;
 
                 for (int j = 0; (j < a.nite) && (fstep > 0); ++j) {  // main.cu:153
-                    double tmin = 2.0;
-                    int hit = -1;
-                    face(0, v0, xt0, g0, tmin, hit);
-                    face(1, v1, xt1, g1, tmin, hit);
-                    face(2, v2, xt2, g2, tmin, hit);
-                    if (tmin < 0.0) break;                          // main.cu:226-229
-
-                    const double st = s_step[ai];                   // main.cu:231-244
-                    if ((fstep * st) >= tmin) {
-                        const double q = tmin / st;
-                        fstep = fstep - q;
-                        xt0 = xt0 + tmin * v0;
-                        xt1 = xt1 + tmin * v1;
-                        xt2 = xt2 + tmin * v2;
-                        add_residence(tc, ai, q);
-                    } else {
-                        const double f = st * fstep;
-                        xt0 = xt0 + f * v0;
-                        xt1 = xt1 + f * v1;
-                        xt2 = xt2 + f * v2;
-                        add_residence(tc, ai, fstep);
+                    const double d0 = f0 - xt0, d1 = f1 - xt1, d2 = f2 - xt2;
+                    const double u0 = d0 * y0, u1 = d1 * y1, u2 = d2 * y2;
+                    const bool b1 = u1 < u0;
+                    const double lo = b1 ? u1 : u0, hi = b1 ? u0 : u1;
+                    const bool b2 = u2 < lo;
+                    double tmin = b2 ? u2 : lo;
+                    const double next = b2 ? lo : (u2 < hi ? u2 : hi);
+                    int hit = b2 ? 2 : (b1 ? 1 : 0);
+                    const double st_ = s_step[ai];                  // main.cu:231-244
+                    const double reach = fstep * st_;
+                    bool ends = reach * kNear < tmin;
+                    if (!ends) {
+                        tmin = tmin > 0.0 ? tmin : 0.0;
+                        if (reach > tmin * kNear && next > tmin * kNear) {
+                            const double d = hit == 0 ? d0 : (hit == 1 ? d1 : d2);
+                            const double v = hit == 0 ? v0 : (hit == 1 ? v1 : v2);
+                            const double y = hit == 0 ? y0 : (hit == 1 ? y1 : y2);
+                            const double q = div_by(d, v, y);
+                            tmin = (0.0 < q) ? q : 0.0;
+                        } else {
+                            // too close to call: the exact quotients, lowest axis on ties
+                            tmin = 2.0;
+                            hit = -1;
+                            const double t0 = face_time(d0, v0), t1 = face_time(d1, v1), t2 = face_time(d2, v2);
+                            if (t0 < tmin) { tmin = t0; hit = 0; }
+                            if (t1 < tmin) { tmin = t1; hit = 1; }
+                            if (t2 < tmin) { tmin = t2; hit = 2; }
+                            ends = !(reach >= tmin);
+                        }
+                    }
+                    if (ends) {
+                        xt0 = xt0 + reach * v0;
+                        xt1 = xt1 + reach * v1;
+                        xt2 = xt2 + reach * v2;
+                        tcur = tcur + fstep;
                         fstep = 0.0;
                         break;
                     }
+                    const double q = div_by(tmin, st_, s_rstep[ai]);
+                    fstep = fstep - q;
+                    xt0 = xt0 + tmin * v0;
+                    xt1 = xt1 + tmin * v1;
+                    xt2 = xt2 + tmin * v2;
+                    tcur = tcur + q;
                     if (hit < 0) { atomicOr(a.err, kErrStep); break; }
 
                     // neighbour voxel; lattice wall (main.cu:246-265)
-                    const double vh = hit == 0 ? v0 : (hit == 1 ? v1 : v2);
-                    const int gh = hit == 0 ? g0 : (hit == 1 ? g1 : g2);
-                    const int nh = hit == 0 ? a.n1 : (hit == 1 ? a.n2 : a.n3);
-                    int gj = (vh >= 0.0) ? gh + 1 : gh - 1;
-                    const int wall = (gj >= nh) ? 1 : ((gj < 0) ? -1 : 0);
-                    if (wall != 0 && mirror) {
-                        if (wall > 0) f1 |= 1u << hit; else f0 |= 1u << hit;
-                        if (hit == 0) v0 = -v0; else if (hit == 1) v1 = -v1; else v2 = -v2;
-                        ev |= ((1u << 2) | (uint32_t)hit) << (4 * nev++);
-                        continue;
-                    }
-                    if (wall != 0) gj = (wall > 0) ? 0 : nh - 1;   // periodic neighbour
-
-                    // membrane (main.cu:272-289)
-                    const int j0 = hit == 0 ? gj : g0;
-                    const int j1 = hit == 1 ? gj : g1;
-                    const int j2 = hit == 2 ? gj : g2;
-                    const int aj = (int)__ldg(a.labels + lin3(j0, j1, j2, a.n2, a.n3));
-                    const double P = s_pij[ai * a.nc + aj];
-                    bool cross;
-                    if (P > 0.999999) {
-                        cross = true;
-                    } else if (P < 0.000001) {
-                        cross = false;
+                    const bool up = (ups >> hit) & 1u;
+                    const double fh = hit == 0 ? f0 : (hit == 1 ? f1 : f2);
+                    const double nh = hit == 0 ? n0 : (hit == 1 ? n1 : n2);
+                    const int lh = hit == 0 ? l0 : (hit == 1 ? l1 : 1);
+                    const bool wall = up ? fh >= nh : fh <= 0.0;
+                    bool cross = false;
+                    int aj = ai, lj = lin;
+                    if (wall && mirror) {
+                        if (up) wall1 |= 1u << hit; else wall0 |= 1u << hit;
+                        if (TRACE) ev |= ((1u << 2) | (uint32_t)hit) << (4 * nev++);
                     } else {
-                        cross = rng.next() < P;
+                        // membrane (main.cu:272-289); a periodic wall's neighbour is on the far side
+                        if (!wall) lj += up ? lh : -lh;
+                        else lj += up ? -((int)nh - 1) * lh : ((int)nh - 1) * lh;
+                        aj = (int)__ldg(a.labels + (unsigned)lj);
+                        const double P = s_pij[ai * a.nc + aj];
+                        if (P > 0.999999) {
+                            cross = true;
+                        } else if (P < 0.000001) {
+                            cross = false;
+                        } else {
+                            cross = rng.next() < P;
+                        }
+                        if (TRACE)
+                            ev |= (((cross ? (wall ? 1u : 3u) : 2u) << 2) | (uint32_t)hit) << (4 * nev++);
                     }
+                    // the face ahead next: a voxel further on, or the one behind after a reflection
+                    double df = up ? 1.0 : -1.0;
                     if (cross) {
-                        ai = aj;
-                        g0 = j0; g1 = j1; g2 = j2;
-                        if (wall != 0) {
-                            const double shift = (wall > 0) ? -(double)nh : (double)nh;
+                        if (aj != ai) {
+                            s_tc[ai][threadIdx.x] = tcur;
+                            tcur = s_tc[aj][threadIdx.x];
+                            ai = aj;
+                        }
+                        lin = lj;
+                        if (wall) {
+                            const double shift = up ? -nh : nh;
+                            df = df + shift;
                             if (hit == 0) { xt0 = xt0 + shift; xi0 = xi0 + shift; }
                             else if (hit == 1) { xt1 = xt1 + shift; xi1 = xi1 + shift; }
                             else { xt2 = xt2 + shift; xi2 = xi2 + shift; }
-                            ev |= ((1u << 2) | (uint32_t)hit) << (4 * nev++);
-                        } else {
-                            ev |= ((3u << 2) | (uint32_t)hit) << (4 * nev++);
                         }
                     } else {
-                        if (hit == 0) v0 = -v0; else if (hit == 1) v1 = -v1; else v2 = -v2;
-                        ev |= ((2u << 2) | (uint32_t)hit) << (4 * nev++);
+                        df = -df;
+                        ups ^= 1u << hit;
+                        if (hit == 0) { v0 = -v0; y0 = -y0; }
+                        else if (hit == 1) { v1 = -v1; y1 = -y1; }
+                        else { v2 = -v2; y2 = -y2; }
                     }
+                    if (hit == 0) f0 = f0 + df; else if (hit == 1) f1 = f1 + df; else f2 = f2 + df;
                 }
-                if (fstep > 0) ev |= 1u << 31;
-                ev |= (uint32_t)nev << 28;
+                g0 = (ups & 1u) ? f0 - 1.0 : f0;
+                g1 = (ups & 2u) ? f1 - 1.0 : f1;
+                g2 = (ups & 4u) ? f2 - 1.0 : f2;
 
                 // mirror the origin for each wall hit this step (main.cu:302-310)
-                if (f0 & 1u) xi0 = -xi0;
-                if (f1 & 1u) xi0 = 2.0 * (double)a.n1 - xi0;
-                if (f0 & 2u) xi1 = -xi1;
-                if (f1 & 2u) xi1 = 2.0 * (double)a.n2 - xi1;
-                if (f0 & 4u) xi2 = -xi2;
-                if (f1 & 4u) xi2 = 2.0 * (double)a.n3 - xi2;
+                if (wall0 | wall1) {
+                    if (wall0 & 1u) xi0 = -xi0;
+                    if (wall1 & 1u) xi0 = 2.0 * n0 - xi0;
+                    if (wall0 & 2u) xi1 = -xi1;
+                    if (wall1 & 2u) xi1 = 2.0 * n1 - xi1;
+                    if (wall0 & 4u) xi2 = -xi2;
+                    if (wall1 & 4u) xi2 = 2.0 * n2 - xi2;
+                }
                 if (TRACE && w < a.trace_n) {
-                    a.tr_vox[(size_t)w * a.tn + i] = (int32_t)lin3(g0, g1, g2, a.n2, a.n3);
+                    if (fstep > 0) ev |= 1u << 31;
+                    ev |= (uint32_t)nev << 28;
+                    a.tr_vox[(size_t)w * a.tn + i] = lin;
                     a.tr_ev[(size_t)w * a.tn + i] = ev;
                     double* tp = a.tr_pos + ((size_t)w * a.tn + i) * 3;
                     tp[0] = xt0; tp[1] = xt1; tp[2] = xt2;
                 }
             }
 
-            if (pgse) {
+            if (PGSE) {
                 // displacement of this step's position (main_PGSE.cu:336-338)
                 p0 = p0 + (xt0 - xi0) * a.res;
                 p1 = p1 + (xt1 - xi1) * a.res;
@@ -245,108 +402,67 @@ __global__ void __launch_bounds__(kBlock) walk_compat_kernel(const WalkArgs a) {
                     } while (evi < a.nevents && a.ev_step[evi] == i + 1);
                     next_ev = (evi < a.nevents) ? a.ev_step[evi] : -1;
                 }
-                if (i == a.tn - 1) {
-                    // final T2-weighted signal (main_PGSE.cu:348-357)
-                    double s0 = 0.0;
-#pragma unroll
-                    for (int c = 0; c < NCMAX; ++c)
-                        if (c < a.nc) s0 = s0 + tc[c] / s_t2[c];
-                    s0 = active ? exp(-1.0 * s0) : 0.0;
-                    for (int base = 0; base < a.ngrad; base += 32) {
-                        double mine = 0.0;
-                        const int cnt = min(32, a.ngrad - base);
-                        for (int k = 0; k < cnt; ++k) {
-                            const int jg = base + k;
-                            const double* vv = a.vscr + (size_t)(a.gpair[jg] * 3) * nthr + gtid;
-                            const double* g = a.grad + 6 * jg;
-                            const double phase =
-                                g[2] * (vv[0] * g[3] + vv[nthr] * g[4] + vv[2 * (size_t)nthr] * g[5]) * a.dt;
-                            const double r = warp_sum(s0 * cos(phase));
-                            if (lane == k) mine = r;
-                        }
-                        if (lane < cnt) sig_slot[base + lane] += mine;
-                    }
-                }
             }
 
             // record every tstep steps (main.cu:333-379; i % tstep == 0 as a countdown)
             if (i == next_rec) {
-                const int tidx = rec++;
-                next_rec += a.tstep;
-                if (tidx < a.timepoints) {
-                    double s0 = 0.0;
-#pragma unroll
-                    for (int c = 0; c < NCMAX; ++c)
-                        if (c < a.nc) s0 = s0 + tc[c] / s_t2[c];
-                    s0 = active ? exp(-1.0 * s0) : 0.0;
-                    const double dx = (xt0 - xi0) * a.res;
-                    const double dy = (xt1 - xi1) * a.res;
-                    const double dz = (xt2 - xi2) * a.res;
-                    double v[32];
-                    v[0] = s0;
-                    v[1] = s0 * dx * dx;  v[2] = s0 * dx * dy;  v[3] = s0 * dx * dz;
-                    v[4] = s0 * dy * dy;  v[5] = s0 * dy * dz;  v[6] = s0 * dz * dz;
-                    v[7] = s0 * dx * dx * dx * dx;   v[8] = s0 * dx * dx * dx * dy;
-                    v[9] = s0 * dx * dx * dx * dz;   v[10] = s0 * dx * dx * dy * dy;
-                    v[11] = s0 * dx * dx * dy * dz;  v[12] = s0 * dx * dx * dz * dz;
-                    v[13] = s0 * dx * dy * dy * dy;  v[14] = s0 * dx * dy * dy * dz;
-                    v[15] = s0 * dx * dy * dz * dz;  v[16] = s0 * dx * dz * dz * dz;
-                    v[17] = s0 * dy * dy * dy * dy;  v[18] = s0 * dy * dy * dy * dz;
-                    v[19] = s0 * dy * dy * dz * dz;  v[20] = s0 * dy * dz * dz * dz;
-                    v[21] = s0 * dz * dz * dz * dz;
-#pragma unroll
-                    for (int c = 0; c < 10; ++c) v[kColCount + c] = (active && ai == c) ? 1.0 : 0.0;
-                    const double r = warp_reduce_scatter32(v, lane);
-                    double* row = slot + (size_t)tidx * a.nvals;
-                    row[lane] += r;
-                    if (!pgse) {
-                        // narrow-pulse signal (main.cu:374-378)
-                        for (int base = 0; base < a.nbvec; base += 32) {
-                            double mine = 0.0;
-                            const int cnt = min(32, a.nbvec - base);
-                            for (int k = 0; k < cnt; ++k) {
-                                const int jb = base + k;
-                                const double qx = a.qtab[(size_t)tidx * a.nbvec + jb] *
-                                                  (dx * a.bvec[jb * 3 + 0] + dy * a.bvec[jb * 3 + 1] +
-                                                   dz * a.bvec[jb * 3 + 2]);
-                                const double rr = warp_sum(s0 * cos(qx));
-                                if (lane == k) mine = rr;
-                            }
-                            if (lane < cnt) row[kRowHead + base + lane] += mine;
-                        }
-                    }
+                const int r = rec & (kRec - 1), rec0 = rec - r;   // slot in the batch, the batch's first record
+                ++rec;
+                next_rec = rec < a.timepoints ? next_rec + a.tstep : -1;
+                double* mine = st + r * kStageRow + lane;
+                mine[0] = (xt0 - xi0) * a.res;
+                mine[32] = (xt1 - xi1) * a.res;
+                mine[64] = (xt2 - xi2) * a.res;
+                mine[96] = weight();
+                const unsigned b0 = __ballot_sync(0xffffffffu, ai & 1), b1 = __ballot_sync(0xffffffffu, ai & 2),
+                               b2 = __ballot_sync(0xffffffffu, ai & 4);
+                if (lane < 3) stage_masks(st + r * kStageRow)[lane] = lane == 0 ? b0 : (lane == 1 ? b1 : b2);
+                if (r == kRec - 1 || rec == a.timepoints) {
+                    const unsigned act = __ballot_sync(0xffffffffu, active);
+                    double* row = slot + (size_t)rec0 * a.nvals;
+                    add_moments(st, row, a.nvals, rec - rec0, act, a.tile_w, first, lane);
+                    if (!PGSE && a.nbvec > 0)
+                        add_signals(st, a.qtab + (size_t)rec0 * a.nbvec, a.bvec, a.nbvec, row + kRowHead, a.nvals,
+                                    rec - rec0, a.tile_w, first, lane);
+                    __syncwarp();
                 }
             }
         }
+        if (PGSE)
+            add_pgse(a, nthr, gtid - lane, weight(), a.tile_w, a.sig_slots + (size_t)warp_global * a.ngrad_pad, first,
+                     lane);
     }
 }
 
-template <int NCMAX, bool TRACE>
-int launch_t(const WalkArgs& a, int grid, int block, void* stream) {
-    walk_compat_kernel<NCMAX, TRACE><<<grid, block, 0, (cudaStream_t)stream>>>(a);
-    return (int)cudaGetLastError();
+template <class F>
+auto by_form(int nc, bool trace, bool pgse, int minb, F&& f) {
+    auto blocks = [&]<int NC, bool PG>() {
+        if (trace) return f.template operator()<NC, true, PG, 4>();
+        if (minb == 6) return f.template operator()<NC, false, PG, 6>();
+        if (minb == 5) return f.template operator()<NC, false, PG, 5>();
+        return f.template operator()<NC, false, PG, 4>();
+    };
+    if (nc <= 4) return pgse ? blocks.template operator()<4, true>() : blocks.template operator()<4, false>();
+    return pgse ? blocks.template operator()<8, true>() : blocks.template operator()<8, false>();
 }
 
 }  // namespace
 
-int launch_walk_compat(const WalkArgs& a, int grid, int block, bool trace, void* stream) {
+int launch_walk_compat(const WalkArgs& a, int grid, int block, int minb, bool trace, void* stream) {
     if (block != kBlock) return (int)cudaErrorInvalidValue;
-    if (a.nc <= 4) return trace ? launch_t<4, true>(a, grid, block, stream)
-                                : launch_t<4, false>(a, grid, block, stream);
-    return trace ? launch_t<8, true>(a, grid, block, stream)
-                 : launch_t<8, false>(a, grid, block, stream);
+    return by_form(a.nc, trace, a.mode == 1, minb, [&]<int NC, bool TR, bool PG, int MB>() {
+        walk_compat_kernel<NC, TR, PG, MB><<<grid, kBlock, 0, (cudaStream_t)stream>>>(a);
+        return (int)cudaGetLastError();
+    });
 }
 
-int walk_compat_blocks_per_sm(int nc, bool trace) {
-    int n = 0;
-    cudaError_t e;
-    if (nc <= 4)
-        e = trace ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_compat_kernel<4, true>, kBlock, 0)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_compat_kernel<4, false>, kBlock, 0);
-    else
-        e = trace ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_compat_kernel<8, true>, kBlock, 0)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_compat_kernel<8, false>, kBlock, 0);
-    return e == cudaSuccess ? n : -1;
+int walk_compat_blocks_per_sm(int nc, bool trace, bool pgse, int minb) {
+    return by_form(nc, trace, pgse, minb, [&]<int NC, bool TR, bool PG, int MB>() {
+        int n = 0;
+        const cudaError_t e =
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_compat_kernel<NC, TR, PG, MB>, kBlock, 0);
+        return e == cudaSuccess ? n : -1;
+    });
 }
 
 }  // namespace rms
