@@ -124,7 +124,8 @@ size_t padded_lattice_bytes(int n1, int n2, int n3, int bits);
 // mirror: flag voxels at the lattice's faces too (mirror walls; see pad_pack_kernel)
 int pack_lattice_padded(const uint8_t* labels, int n1, int n2, int n3, int bits, int mirror, uint8_t* out,
                         void* stream);
-int launch_reduce_slots(const double* slots, int nslots, size_t row, double* out, void* stream);
+// (the rows are overwritten)
+int launch_reduce_slots(double* slots, int nslots, size_t row, double* out, void* stream);
 // Resident blocks per SM of the walk kernels (occupancy API); -1 on error.
 // (minb: the COMPAT walk's form, built for 4, 5 or 6 resident blocks)
 int walk_compat_blocks_per_sm(int nc, bool trace, bool pgse, int minb);
