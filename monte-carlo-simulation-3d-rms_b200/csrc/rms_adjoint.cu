@@ -82,6 +82,33 @@ __device__ __forceinline__ float warp_reduce_scatter16f(float (&v)[16], int lane
     return v[0];
 }
 
+// The waveform tables of one bin, [waveform][axis] as doubles and the float4
+// pairs of AdjArgs::wq, for one warp: fetched asynchronously while the bin is
+// walked, read as broadcasts at its end.  Reading them from global memory there
+// cost a warp one L2 latency per waveform (the tables of 1000 bins do not stay
+// in L1): 16 of them a bin, most of the pass.
+struct BinTables {
+    double g[kAdjWaves * 3];
+    float4 q[kAdjWaves * 2];
+};
+__device__ __forceinline__ void fetch_bin(BinTables& t, const AdjArgs& a, int bin, int lane, bool floats) {
+    __syncwarp();   // the last bin's tables have been read
+    if (bin >= a.nbins) return;
+    const double* g = a.wave + (size_t)bin * a.nwave * 3;
+    for (int e = lane; e < 3 * a.nwave; e += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(t.g + e)),
+                     "l"(g + e)
+                     : "memory");
+    if (floats && lane < 2 * a.nwave)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(t.q + lane)),
+                     "l"(a.wq + (size_t)bin * a.nwave * 2 + lane)
+                     : "memory");
+}
+__device__ __forceinline__ void bin_ready() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+}
+
 // What pass 1 records during a step (split_step's hooks): the path per
 // compartment, the displacement's tangent with respect to the step length
 // (flipped at every reflection) and the permeation score.
@@ -134,18 +161,18 @@ struct LaneArr {
     __device__ __forceinline__ float& operator[](int j) const { return p[j * kAdjBlock]; }
 };
 
-// Resident blocks per SM: at least 5 for the weighted-loss form (96 registers,
-// no spills); the Jacobian form takes the compiler's choice (123 registers, 4
-// blocks) except FORMs 1 and 2, held to 4 blocks (unbounded they took 248 and
-// 134 registers).  FORM 1 of the weighted form also runs at 4 blocks: at 5
-// (96 registers, 116 bytes spilled) the job below took 175 ms, at 4 (128
-// registers, 48 bytes) 155 ms.
-// Measured on a 64x64x512 axon, 1e6 walkers x 5000 steps, 16 waveforms, all
-// passes in one launch: weighted 428 ms (518 ms at 4 blocks), Jacobian 390 ms
-// (416 ms when held to 4 blocks at 115 registers); with the per-lane arrays
-// in registers (3 blocks) 541 / 474 ms.  FORM 1, the dL/dwave reduction and
-// FORM 2 (11 resume steps 480 steps apart): 155 / 149 ms (forward walk 154 ms;
-// with pass 2 still walked and the forced walks grouped, 310 / 308 ms).
+// Resident blocks per SM.  What the walks wait for is the label gathers (long
+// scoreboard), so they want warps and L1: the per-lane arrays a form does not
+// read back are not kept (28 KB a block in FORM 1, 12 / 20 KB in FORM 2, where
+// all forms once held 25-33 KB), and the waveform tables are fetched into
+// shared memory while the bin is walked.  With that FORM 1 runs 6 blocks (80
+// registers, 16 bytes spilled) and FORM 2 5 (96 registers, none); 7 or 8 blocks
+// spill and take the L1.  FORM 0: 5 for the weighted loss, the compiler's choice
+// for the Jacobian.
+// Measured on a 64x64x512 axon, 5000 steps, 1000 bins, 16 waveforms (weighted /
+// Jacobian): 1e5 walkers 24.5 / 23.2 -> 19.7 / 19.7 ms, 4e5 walkers 66.4 / 64.1
+// -> 57.4 / 57.9 ms (FORM 1 at 4 blocks: 24.5 and 65.9; 5: 25.1 and 60.6; 7:
+// 22.6 and 66.6).
 //
 // FORM 0 walks all passes in this launch.  FORM 1 walks pass 1 only and
 // leaves in memory what passes 2 and 3 need: the bin displacement sums X_wb
@@ -159,15 +186,20 @@ struct LaneArr {
 // warp, each from its checkpoint -- so a warp no longer walks from step 0
 // because one lane's draw came early.  The sums are the single launch's up to
 // the order of the float and FP64 sums.
-constexpr int adj_min_blocks(bool jac, int form) { return form == 1 ? 4 : (jac ? (form == 2 ? 4 : 1) : 5); }
+constexpr int adj_min_blocks(bool jac, int form) { return form == 1 ? 6 : (form == 2 ? 5 : (jac ? 1 : 5)); }
 
 template <bool JAC, int FORM>
 __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_kernel(const __grid_constant__ AdjArgs a) {
     constexpr int NC = kAdjNc, BITS = 4, NW = kAdjWaves;
     constexpr int kTab = 2 * NC + 2 * NC * NC;
     __shared__ float s_tab[kTab];
-    // per lane: phi, dphi, aj (LaneArr); FORM 1: + the time-rescaling sums R_j
-    __shared__ float s_lane[FORM == 1 ? 4 : 3][NW][kAdjBlock];
+    // per lane (LaneArr): phi; dphi but in the weighted FORM 2; and a_jw (FORM 0)
+    // or the time-rescaling sums R_j (FORM 1, whose a_jw live one j at a time).
+    // What is not kept here is L1 for the label gathers.
+    constexpr int kLane = FORM == 2 ? (JAC ? 2 : 1) : 3;
+    __shared__ float s_lane[kLane][NW][kAdjBlock];
+    __shared__ __align__(16) BinTables s_bin[kAdjBlock / 32];
+    BinTables& tab_b = s_bin[threadIdx.x >> 5];
     for (int i = threadIdx.x; i < kTab; i += blockDim.x)
         s_tab[i] = i < NC ? a.step[i]
                           : (i < 2 * NC ? a.kexp[i - NC]
@@ -211,13 +243,12 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
         }
         w = a.walker_begin + wr;
         const uint32_t wlo = (uint32_t)w, whi = (uint32_t)((uint64_t)w >> 32);
-        const LaneArr phi{&s_lane[0][0][threadIdx.x]}, dphi{&s_lane[1][0][threadIdx.x]}, aj{&s_lane[2][0][threadIdx.x]};
-        const LaneArr rr{&s_lane[FORM == 1 ? 3 : 0][0][threadIdx.x]};   // FORM 1 only
+        const LaneArr phi{&s_lane[0][0][threadIdx.x]}, dphi{&s_lane[kLane > 1 ? 1 : 0][0][threadIdx.x]};
+        const LaneArr aj{&s_lane[kLane - 1][0][threadIdx.x]}, rr = aj;   // FORM 0's a_jw, FORM 1's R_j
 #pragma unroll
-        for (int j = 0; j < NW; ++j) phi[j] = dphi[j] = aj[j] = 0.0f;
-        if (FORM == 1) {
+        for (int j = 0; j < NW; ++j) {
 #pragma unroll
-            for (int j = 0; j < NW; ++j) rr[j] = 0.0f;
+            for (int k = 0; k < kLane; ++k) s_lane[k][j][threadIdx.x] = 0.0f;
         }
         AdjHooks<NC> h;
 #pragma unroll
@@ -326,6 +357,7 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
             }
             float B0 = 0.0f, B1 = 0.0f, B2 = 0.0f;  // bin sums of the tangent
             int bin = i_start / a.bin_steps, next_bin = (i_start / a.bin_steps + 1) * a.bin_steps;
+            fetch_bin(tab_b, a, bin, lane, pass < 2);
             float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f, q3 = 0.0f;   // the split walk's direction stream
             int phase = 0;
             uint32_t dblk = (uint32_t)(i_start / 3);
@@ -393,19 +425,20 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                 }
                 if (event) {
                     const double x0 = P0 * (double)a.res, x1 = P1 * (double)a.res, x2 = P2 * (double)a.res;
-                    const double* wv = a.wave + (size_t)bin * a.nwave * 3;
-                    const float4* wq = a.wq + (size_t)bin * a.nwave * 2;   // [j]: g_j,b - g_j,b+1; g_j,b res
+                    bin_ready();
+                    const double* wv = tab_b.g;
+                    const float4* wq = tab_b.q;   // [j]: g_j,b - g_j,b+1; g_j,b res
                     if (pass != 1) {
                         // the phases (pass 1: and their tangents; pass 3: of the forced walk)
 #pragma unroll
                         for (int j = 0; j < NW; ++j) {
                             if (j < a.nwave) {
-                                const double g0 = __ldg(wv + 3 * j), g1 = __ldg(wv + 3 * j + 1), g2 = __ldg(wv + 3 * j + 2);
+                                const double g0 = wv[3 * j], g1 = wv[3 * j + 1], g2 = wv[3 * j + 2];
                                 const float inc = (float)(g0 * x0 + g1 * x1 + g2 * x2);
                                 if (JAC && pass == 2) dphi[j] += inc;
                                 else phi[j] += inc;
                                 if (p1st) {
-                                    const float4 gr = __ldg(wq + 2 * j + 1);
+                                    const float4 gr = wq[2 * j + 1];
                                     dphi[j] += fmaf(gr.z, B2, fmaf(gr.y, B1, gr.x * B0));
                                 }
                             }
@@ -427,7 +460,7 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
 #pragma unroll
                             for (int j = 0; j < NW; ++j) {
                                 if (j < a.nwave) {
-                                    const float4 q = __ldg(wq + 2 * j);
+                                    const float4 q = wq[2 * j];
                                     rr[j] = fmaf(tb, q.x * xe0 + q.y * xe1 + q.z * xe2, rr[j]);
                                 }
                             }
@@ -441,7 +474,7 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
 #pragma unroll
                         for (int j = 0; j < NW; ++j) {
                             if (j < a.nwave) {
-                                const float4 q = __ldg(wq + 2 * j);
+                                const float4 q = wq[2 * j];
                                 if (JAC) dphi[j] = fmaf(tb, q.x * xe0 + q.y * xe1 + q.z * xe2, dphi[j]);   // R_j
                                 else tr = fmaf(aj[j] * tb, q.x * xe0 + q.y * xe1 + q.z * xe2, tr);
                             }
@@ -462,6 +495,7 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                     P0 = P1 = P2 = 0.0;
                     ++bin;
                     next_bin += a.bin_steps;
+                    fetch_bin(tab_b, a, bin, lane, pass < 2);
                 }
             }
             w64 += (double)wk.w32;
@@ -480,12 +514,13 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                         gs = __ldg(a.gup + 2 * j + 1);
                     }
                     Lw += s0w * (gc * cs + gs * sn);
-                    aj[j] = s0w * (gs * cs - gc * sn);
-                    G += aj[j] * dphi[j];
-                    tr -= aj[j] * phi[j];
+                    const float ajw = s0w * (gs * cs - gc * sn);
+                    if (FORM == 0) aj[j] = ajw;
+                    G += ajw * dphi[j];
+                    tr -= ajw * phi[j];
                     if (FORM == 1 && !JAC && j < a.nwave) {
-                        tr = fmaf(aj[j], rr[j], tr);   // pass 2's time-rescaling sum
-                        if (live) a.ajw[(size_t)j * a.nwalk + wr] = aj[j];
+                        tr = fmaf(ajw, rr[j], tr);   // pass 2's time-rescaling sum
+                        if (live) a.ajw[(size_t)j * a.nwalk + wr] = ajw;
                     }
                     const double C = warp_sum((double)(s0w * cs)), S = warp_sum((double)(s0w * sn));
                     if (lane == 0 && j < a.nwave) {
