@@ -749,6 +749,8 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
     a.traj = traj;
     a.traj_split = (o && o->traj_split) ? 1 : 0;
     a.traj_n = jobs[0].w1 - jobs[0].w0;
+    // eight bins are 96 (48 + 48) bytes: on 16-byte boundaries when the rows hold whole eights and the buffer is
+    a.traj_vec = (wavemode && s->nbins % 8 == 0 && reinterpret_cast<uintptr_t>(traj) % 16 == 0) ? 1 : 0;
     a.rows = d->rows.as<double>();
     a.tpad = tpad;
     a.nb_pad = nb_pad;

@@ -93,6 +93,7 @@ struct WalkArgs {
     const double* wave;
     float* traj;
     int traj_split;             // traj holds BF16 hi parts, then lo parts (per walker, bin, axis)
+    int traj_vec;               // its rows can be written 8 bins at a time in 16-byte stores
     int64_t traj_n;             // walkers in the trajectory buffer
     AxonDesc axon0;             // the first axon, by value (read from kernel parameters)
     // traces (COMPAT)

@@ -69,29 +69,83 @@ constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 // General waveforms, at the end of bin `bin`: X (voxels) is the bin's
 // displacement sum; every waveform's phase gets wave_b . X res, and the bin's
 // mean displacement (um) goes to the trajectory output when one is given.
+//
+// Waveforms go four at a time: a phase is read from and written to the thread's
+// scratch in L2, and one at a time each waited out that latency alone.  A
+// trajectory row is 12 bytes a bin, one row per lane: written bin by bin, every
+// store touched 32 sectors for a few bytes each, so kTrajBins bins wait in
+// `wait` (local memory) and leave as 16-byte stores where rows are 16-byte
+// aligned (traj_vec).
+constexpr int kTrajBins = 8;
 __device__ __noinline__ void wave_bin(const double* __restrict__ wave, int nwave, int bin, double X0, double X1,
                                       double X2, double res, double* ph, int nthr, float* traj, int64_t tw,
-                                      int nbins, int bin_steps, int split, int64_t traj_n) {
+                                      int nbins, int bin_steps, int split, int vec, int64_t traj_n, uint32_t* wait) {
     const double x0 = X0 * res, x1 = X1 * res, x2 = X2 * res;
     const double* wv = wave + (size_t)bin * nwave * 3;
-    for (int j = 0; j < nwave; ++j) ph[(size_t)j * nthr] += wv[3 * j] * x0 + wv[3 * j + 1] * x1 + wv[3 * j + 2] * x2;
-    if (traj && tw >= 0) {
-        const double inv = 1.0 / (double)bin_steps;
-        const float m[3] = {(float)(x0 * inv), (float)(x1 * inv), (float)(x2 * inv)};
-        const size_t at = ((size_t)tw * nbins + bin) * 3;
+    int j = 0;
+    for (; j + 4 <= nwave; j += 4) {
+        double p[4], g[12];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) p[q] = ph[(size_t)(j + q) * nthr];
+#pragma unroll
+        for (int q = 0; q < 12; ++q) g[q] = __ldg(wv + 3 * j + q);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) p[q] += g[3 * q] * x0 + g[3 * q + 1] * x1 + g[3 * q + 2] * x2;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ph[(size_t)(j + q) * nthr] = p[q];
+    }
+    for (; j < nwave; ++j) ph[(size_t)j * nthr] += wv[3 * j] * x0 + wv[3 * j + 1] * x1 + wv[3 * j + 2] * x2;
+    if (!traj || tw < 0) return;
+    const double inv = 1.0 / (double)bin_steps;
+    const float m[3] = {(float)(x0 * inv), (float)(x1 * inv), (float)(x2 * inv)};
+    const size_t at = ((size_t)tw * nbins + bin) * 3;
+    // split: BF16 pairs, hi = bf16(x), lo = bf16(x - hi): the operands of the
+    // tensor-core contraction, split once here
+    uint32_t word[3];   // hi | lo << 16
+    if (split) {
+        for (int k = 0; k < 3; ++k) {
+            const __nv_bfloat16 h = __float2bfloat16_rn(m[k]);
+            const __nv_bfloat16 l = __float2bfloat16_rn(m[k] - __bfloat162float(h));
+            word[k] = (uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(l) << 16);
+        }
+    } else {
+        for (int k = 0; k < 3; ++k) word[k] = __float_as_uint(m[k]);
+    }
+    if (!vec) {
         if (split) {
-            // BF16 pairs, hi = bf16(x), lo = bf16(x - hi): the operands of the
-            // tensor-core contraction, split once here
-            __nv_bfloat16* hi = reinterpret_cast<__nv_bfloat16*>(traj);
-            __nv_bfloat16* lo = hi + (size_t)traj_n * nbins * 3;
+            unsigned short* hi = reinterpret_cast<unsigned short*>(traj);
+            unsigned short* lo = hi + (size_t)traj_n * nbins * 3;
             for (int k = 0; k < 3; ++k) {
-                const __nv_bfloat16 h = __float2bfloat16_rn(m[k]);
-                hi[at + k] = h;
-                lo[at + k] = __float2bfloat16_rn(m[k] - __bfloat162float(h));
+                hi[at + k] = (unsigned short)(word[k] & 0xffffu);
+                lo[at + k] = (unsigned short)(word[k] >> 16);
             }
         } else {
-            traj[at] = m[0]; traj[at + 1] = m[1]; traj[at + 2] = m[2];
+            for (int k = 0; k < 3; ++k) traj[at + k] = __uint_as_float(word[k]);
         }
+        return;
+    }
+    const int slot = bin % kTrajBins;
+    for (int k = 0; k < 3; ++k) wait[3 * slot + k] = word[k];
+    if (slot != kTrajBins - 1) return;
+    const size_t first = at - 3 * (kTrajBins - 1);   // the batch's first bin
+    uint32_t w[3 * kTrajBins];
+#pragma unroll
+    for (int q = 0; q < 3 * kTrajBins; ++q) w[q] = wait[q];
+    if (split) {
+        uint4* hi = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(traj) + first);
+        uint4* lo = reinterpret_cast<uint4*>(reinterpret_cast<unsigned short*>(traj) + (size_t)traj_n * nbins * 3 + first);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const uint32_t* e = w + 8 * q;
+            hi[q] = make_uint4(__byte_perm(e[0], e[1], 0x5410), __byte_perm(e[2], e[3], 0x5410),
+                               __byte_perm(e[4], e[5], 0x5410), __byte_perm(e[6], e[7], 0x5410));
+            lo[q] = make_uint4(__byte_perm(e[0], e[1], 0x7632), __byte_perm(e[2], e[3], 0x7632),
+                               __byte_perm(e[4], e[5], 0x7632), __byte_perm(e[6], e[7], 0x7632));
+        }
+    } else {
+        uint4* out = reinterpret_cast<uint4*>(traj + first);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) out[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
     }
 }
 
@@ -408,6 +462,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
         int phase = 0;
         uint32_t dblk = 0u;
 
+        uint32_t traj_wait[wave ? 3 * kTrajBins : 1];   // bins of this walker's trajectory not yet written
         for (int i = 0; i < a.tn; ++i) {
             float u1, u2;
             if (phase == 0) {
@@ -460,7 +515,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                 }
                 if (event && wave) {
                     wave_bin(a.wave, a.nwave, evi, P0, P1, P2, (double)AXF(res), a.vscr + gtid, nthr, a.traj,
-                             active ? w - AXF(walker_begin) : -1, a.nbins, a.bin_steps, a.traj_split, a.traj_n);
+                             active ? w - AXF(walker_begin) : -1, a.nbins, a.bin_steps, a.traj_split, a.traj_vec, a.traj_n,
+                             traj_wait);
                     P0 = P1 = P2 = 0.0;
                     ++evi;
                     next_ev += a.bin_steps;
