@@ -32,45 +32,131 @@ constexpr int kSplitVariantDefault = 0;   // 256 threads, >= 4 blocks per SM (64
 constexpr int kMaxGrad = 1 << 16;
 constexpr uint64_t kBatchSeedStep = 0x9E3779B97F4A7C15ull;   // seed of batch member k: seed + k * this
 
-// One device allocation that only grows.
-struct DevBuf {
+// Memory of closed simulations, kept for the next ones.  A program that makes a
+// simulation per call (a fit through torch makes two per iteration) spent 10 to
+// 40 ms of each in cudaMalloc, cudaMallocHost and their frees: a pass of
+// waveform gradients over 1e5 walkers took 48 to 70 ms, 34.5 with the cache.
+//  - bounded: at most kMost bytes of each kind, a block that 256 requests in a
+//    row have passed over is freed, and all of them when an allocation fails;
+//  - blocks go to a request they are at most a quarter (and 1 MB) larger than,
+//    on their own device;
+//  - one mutex; a block enters only after the device has finished everything
+//    (what cudaFree would have waited for), so the next owner may use any stream.
+class BlockCache {
+  public:
+    explicit BlockCache(bool host) : host_(host), most_(host ? (size_t)256 << 20 : (size_t)4 << 30) {}
+
+    cudaError_t take(size_t bytes, int device, void** p, size_t* got) {
+        std::lock_guard<std::mutex> lk(mu_);
+        ++now_;
+        int best = -1;
+        for (int k = 0; k < (int)free_.size(); ++k) {
+            const Block& b = free_[k];
+            if (b.device == device && b.n >= bytes && b.n <= bytes + bytes / 4 + ((size_t)1 << 20) &&
+                (best < 0 || b.n < free_[best].n))
+                best = k;
+        }
+        if (best >= 0) {
+            *p = free_[best].p;
+            *got = free_[best].n;
+            held_ -= free_[best].n;
+            free_.erase(free_.begin() + best);
+            return cudaSuccess;
+        }
+        cudaError_t e = host_ ? cudaMallocHost(p, bytes) : cudaMalloc(p, bytes);
+        if (e != cudaSuccess && !free_.empty()) {
+            (void)cudaGetLastError();   // a failed allocation is not sticky; clear it
+            drop([](const Block&) { return true; });
+            e = host_ ? cudaMallocHost(p, bytes) : cudaMalloc(p, bytes);
+        }
+        if (e != cudaSuccess) *p = nullptr;
+        *got = bytes;
+        return e;
+    }
+
+    // the caller's device is the block's
+    void give(void* p, size_t n, int device) {
+        if (cudaDeviceSynchronize() != cudaSuccess || n > most_) {
+            free_block(p);
+            return;
+        }
+        std::lock_guard<std::mutex> lk(mu_);
+        try {
+            free_.push_back(Block{p, n, device, now_});
+        } catch (const std::bad_alloc&) {   // (called from destructors and C entries)
+            free_block(p);
+            return;
+        }
+        held_ += n;
+        drop([&](const Block& b) { return now_ - b.since > 256; });
+        while (held_ > most_) {   // the oldest first
+            const long oldest = free_.front().since;
+            bool one = false;
+            drop([&](const Block& b) { return !one && b.since == oldest && (one = true); });
+        }
+    }
+
+  private:
+    struct Block {
+        void* p;
+        size_t n;
+        int device;
+        long since;
+    };
+    void free_block(void* p) { (void)(host_ ? cudaFreeHost(p) : cudaFree(p)); }
+    template <class F>
+    void drop(F which) {
+        for (size_t k = 0; k < free_.size();) {
+            if (which(free_[k])) {
+                free_block(free_[k].p);
+                held_ -= free_[k].n;
+                free_.erase(free_.begin() + k);
+            } else {
+                ++k;
+            }
+        }
+    }
+    const bool host_;
+    const size_t most_;
+    std::mutex mu_;
+    std::vector<Block> free_;   // oldest first
+    size_t held_ = 0;
+    long now_ = 0;
+};
+
+// (never destroyed: the CUDA context may be gone before static destructors run)
+BlockCache& block_cache(bool host) {
+    static BlockCache* dev = new BlockCache(false);
+    static BlockCache* pinned = new BlockCache(true);
+    return host ? *pinned : *dev;
+}
+
+// One allocation that only grows, on the device or (HOST) pinned.
+template <bool HOST>
+struct Buffer {
     void* p = nullptr;
     size_t n = 0;
+    int device = -1;
     cudaError_t ensure(size_t bytes) {
         if (bytes <= n) return cudaSuccess;
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e == cudaSuccess) n = bytes;
+        release();
+        cudaError_t e = cudaGetDevice(&device);
+        if (e == cudaSuccess) e = block_cache(HOST).take(bytes, device, &p, &n);
+        if (e != cudaSuccess) {
+            p = nullptr;
+            n = 0;
+        }
         return e;
     }
     void release() {
-        if (p) cudaFree(p);
+        if (p) block_cache(HOST).give(p, n, device);
         p = nullptr;
         n = 0;
     }
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
-
-struct HostPinned {
-    void* p = nullptr;
-    size_t n = 0;
-    cudaError_t ensure(size_t bytes) {
-        if (bytes <= n) return cudaSuccess;
-        if (p) cudaFreeHost(p);
-        p = nullptr;
-        n = 0;
-        cudaError_t e = cudaMallocHost(&p, bytes);
-        if (e == cudaSuccess) n = bytes;
-        return e;
-    }
-    void release() {
-        if (p) cudaFreeHost(p);
-        p = nullptr;
-        n = 0;
-    }
-};
+using DevBuf = Buffer<false>;
+using HostPinned = Buffer<true>;
 }  // namespace
 
 struct rms_device_state {
@@ -1224,21 +1310,30 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
     const size_t per_walker =
         (jac ? 0 : sizeof(float) * ((size_t)3 * s->nbins + s->nwave)) +
         (a.force ? sizeof(uint32_t) * ((size_t)kAdjCkWords * (nbk - 1) + kAdjWsWords + nbk) : 0);
-    size_t mfree = 0, mtotal = 0;
-    if (cudaMemGetInfo(&mfree, &mtotal) != cudaSuccess) {
-        (void)cudaGetLastError();
-        mfree = 0;
-    }
-    size_t budget = std::min<size_t>(mfree / 2, (size_t)16 << 30);
+    size_t budget = (size_t)16 << 30;
     if (const char* cap = std::getenv("RMS_ADJOINT_SCRATCH_MB")) {
         const long long mb = std::atoll(cap);
         if (mb > 0) budget = std::min<size_t>(budget, (size_t)mb << 20);
     }
-    int64_t chunk = std::min<int64_t>(nwalk, (int64_t)(budget / std::max<size_t>(per_walker, 1)));
-    if (chunk < nwalk) chunk = chunk / 32 * 32;
+    // half the free memory, asked for when the records are large or do not fit:
+    // cudaMemGetInfo waits for the whole machine's memory calls (0.1 to 20 ms)
+    auto half_free = [] {
+        size_t mfree = 0, mtotal = 0;
+        if (cudaMemGetInfo(&mfree, &mtotal) != cudaSuccess) {
+            (void)cudaGetLastError();
+            mfree = 0;
+        }
+        return mfree / 2;
+    };
     const char* genv = std::getenv("RMS_ADJOINT_GROUPED");
-    bool grouped = !(genv && genv[0] == '0') && chunk >= std::min<int64_t>(nwalk, 65536);
-    if (grouped) {
+    int64_t chunk = 0;
+    bool grouped = false;
+    for (bool asked = std::min(budget, per_walker * (size_t)nwalk) > (size_t)2 << 30;; asked = true) {
+        if (asked) budget = std::min(budget, half_free());
+        chunk = std::min<int64_t>(nwalk, (int64_t)(budget / std::max<size_t>(per_walker, 1)));
+        if (chunk < nwalk) chunk = chunk / 32 * 32;
+        grouped = !(genv && genv[0] == '0') && chunk >= std::min<int64_t>(nwalk, 65536);
+        if (!grouped) break;
         const size_t nwc = (size_t)chunk;
         bool ok = true;
         if (!jac) {
@@ -1251,12 +1346,12 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
             ok = ok && d->adj_blist.ensure(sizeof(int) * (size_t)nbk * nwc) == cudaSuccess;
             ok = ok && d->adj_bcount.ensure(sizeof(int) * kAdjCkMax) == cudaSuccess;
         }
-        if (!ok) {
-            // without room for the records the single launch walks all passes
-            (void)cudaGetLastError();   // a failed allocation is not sticky; clear it
-            for (DevBuf* b : {&d->adj_xbin, &d->adj_ajw, &d->adj_ck, &d->adj_ws, &d->adj_blist}) b->release();
-            grouped = false;
-        }
+        if (ok) break;
+        // without room for the records: smaller chunks, or the single launch that walks all passes
+        (void)cudaGetLastError();   // a failed allocation is not sticky; clear it
+        for (DevBuf* b : {&d->adj_xbin, &d->adj_ajw, &d->adj_ck, &d->adj_ws, &d->adj_blist}) b->release();
+        grouped = false;
+        if (asked) break;
     }
     RMS_CUDA(cudaEventRecord(d->e0, st));
     if (!grouped) {
