@@ -451,7 +451,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
         double w64 = 0.0;          // T2 exponent, folded
         double P0 = 0.0, P1 = 0.0, P2 = 0.0;   // displacement sums (voxels), folded
         float p0 = 0.0f, p1 = 0.0f, p2 = 0.0f;
-        int next_rec = 0, rec = 0;   // the next recorded step (0, tstep, 2 tstep, ...) and its record
+        // records taken, and steps to go to the next one (step 0 is the first) or,
+        // past the last, to the walk's end
+        int rec = 0, left = 1;
         int evi = 0;   // next PGSE event, or current waveform bin
         int next_ev = pgse ? (a.nevents > 0 ? a.ev_step[0] : -1) : (wave ? a.bin_steps : -1);
         if (sums)
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
         uint32_t dblk = 0u;
 
         uint32_t traj_wait[wave ? 3 * kTrajBins : 1];   // bins of this walker's trajectory not yet written
-        for (int i = 0; i < a.tn; ++i) {
+        for (int i = 0;; ++i) {
             float u1, u2;
             if (phase == 0) {
                 float u[6];
@@ -533,10 +535,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                 }
             }
 
-            if (i == next_rec) {
+            if (--left == 0) {
+                if (rec == a.timepoints) break;
                 const int r = rec & (KR - 1), rec0 = rec - r;   // slot in the batch, the batch's first record
                 ++rec;
-                next_rec = rec < a.timepoints ? next_rec + a.tstep : -1;
                 w64 += (double)wk.w32;
                 wk.w32 = 0.0f;
                 const float s0 = active ? expf(-(float)w64) : 0.0f;
@@ -571,6 +573,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                     __syncwarp();
                     unpark_walker(park, wk, perm, q0, q1, q2, q3);
                 }
+                left = rec < a.timepoints ? a.tstep : a.tn - 1 - (rec - 1) * a.tstep;
+                if (left == 0) break;
             }
         }
         if (sums) {

@@ -19,6 +19,31 @@
 
 namespace rms {
 
+// The hardware reciprocal, reciprocal square root, sine and cosine with
+// subnormals flushed: on the walk's arguments (all normal, or zero) the results
+// of __fdividef(1, x), rsqrtf, __sinf and __cosf, without the scaling of
+// subnormal operands around them.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float sin_approx(float x) {
+    float r;
+    asm("sin.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float cos_approx(float x) {
+    float r;
+    asm("cos.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Floor of x in (-1, 2) on the FP32 pipe: x + 1.5 2^23, rounded down, has floor(x)
 // in its low bits and, less 1.5 2^23, as a float (both exact).  FRND and F2I do
 // the same on a pipe of a quarter to an eighth of the rate, which the record
@@ -78,7 +103,6 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
     constexpr int kWall = wall_code<BITS>();
     const uint8_t* __restrict__ lat = g.lat;
     const int s0 = g.s0, s1 = g.s1;
-    const unsigned nu = (v0 > 0.0f ? 1u : 0u) | (v1 > 0.0f ? 2u : 0u) | (v2 > 0.0f ? 4u : 0u);
     // Free flight: a voxel whose 26 neighbours all carry its label has a flag
     // bit; a step from there (shorter than a voxel) moves as one straight line
     // -- the face loop's own outcome, since every face on the way is a
@@ -102,7 +126,7 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
         unsigned lj = (s.lin - g.bias) + __float_as_uint(r0) * (unsigned)s0 + __float_as_uint(r1) * (unsigned)s1 +
                       __float_as_uint(r2);
         unsigned cj = cell_at<BITS>(lat, lj);
-        if ((cj & label_mask<BITS>()) == (unsigned)kWall) {
+        if (cj == (unsigned)kWall) {   // (walls carry no flag)
             int ik0 = (int)k0, ik1 = (int)k1, ik2 = (int)k2;
             // out through one or more mirror walls: reflect on each axis whose
             // face neighbour is a wall (x -> -x below the voxel, 2 - x above)
@@ -141,44 +165,40 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
     // the face loop: up to nite segments, one face event each, on the distances
     // to the next faces along the direction of travel (a face event leaves the
     // walker on the face with a whole voxel ahead: d = 1 exactly)
-    unsigned up = nu;
-    float d0 = (nu & 1u) ? 1.0f - s.o0 : s.o0;
-    float d1 = (nu & 2u) ? 1.0f - s.o1 : s.o1;
-    float d2 = (nu & 4u) ? 1.0f - s.o2 : s.o2;
+    // signed lattice step along each axis in the direction of travel (its sign
+    // is the direction from here on)
+    int dl0 = v0 > 0.0f ? s0 : -s0;
+    int dl1 = v1 > 0.0f ? s1 : -s1;
+    int dl2 = v2 > 0.0f ? 1 : -1;
+    float d0 = v0 > 0.0f ? 1.0f - s.o0 : s.o0;
+    float d1 = v1 > 0.0f ? 1.0f - s.o1 : s.o1;
+    float d2 = v2 > 0.0f ? 1.0f - s.o2 : s.o2;
     const float av0 = fabsf(v0), av1 = fabsf(v1), av2 = fabsf(v2);
-    const float iv0 = __fdividef(1.0f, av0), iv1 = __fdividef(1.0f, av1), iv2 = __fdividef(1.0f, av2);
-    // signed lattice step along each axis in the direction of travel
-    int dl0 = (up & 1u) ? s0 : -s0;
-    int dl1 = (up & 2u) ? s1 : -s1;
-    int dl2 = (up & 4u) ? 1 : -1;
+    const float iv0 = rcp_approx(av0), iv1 = rcp_approx(av1), iv2 = rcp_approx(av2);
     float rem = s.cur_step;        // path left in this step, voxels
     for (int j = 0; j < g.nite; ++j) {
         const float t0 = d0 * iv0, t1 = d1 * iv1, t2 = d2 * iv2;
         const float tm = fminf(t0, fminf(t1, t2));
-        if (rem < tm) {
-            // the step ends inside the voxel
-            d0 = fmaf(-rem, av0, d0); d1 = fmaf(-rem, av1, d1); d2 = fmaf(-rem, av2, d2);
-            s.w32 = fmaf(rem, s.cur_k, s.w32);
-            h.path(s.ai, rem);
-            rem = 0.0f;
-            break;
-        }
-        // onto the nearest face (lowest axis on ties, like the reference's scan)
-        const int hit = (t0 == tm) ? 0 : ((t1 == tm) ? 1 : 2);
-        const float tc = fmaxf(tm, 0.0f);
+        // to the nearest face, or the step's end inside the voxel
+        const bool ends = rem < tm;
+        const float tc = fminf(rem, fmaxf(tm, 0.0f));
         d0 = fmaf(-tc, av0, d0); d1 = fmaf(-tc, av1, d1); d2 = fmaf(-tc, av2, d2);
         s.w32 = fmaf(tc, s.cur_k, s.w32);
         h.path(s.ai, tc);
         rem -= tc;
+        if (ends) break;
+        // (lowest axis on ties, like the reference's scan)
+        const int hit = (t0 == tm) ? 0 : ((t1 == tm) ? 1 : 2);
         const int dl = hit == 0 ? dl0 : (hit == 1 ? dl1 : dl2);
         unsigned lj = s.lin + (unsigned)dl;
-        int aj = label_at<BITS>(lat, lj);
+        unsigned cj = cell_at<BITS>(lat, lj);   // the walker's own cell once it has crossed
+        int aj = (int)(cj & label_mask<BITS>());
         bool cross;
         if (aj == s.ai && g.same_certain) {
             cross = true;
         } else {
             if (aj == kWall) {
-                const bool hi = (up >> hit) & 1u;
+                const bool hi = dl > 0;
                 const int nh = nsize(hit);
                 if (g.mirror) {
                     // mirror wall: reflect, and mirror the origin image
@@ -192,7 +212,8 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
                     // unfolded displacement just continues
                     const int sh = hit == 0 ? s0 : (hit == 1 ? s1 : 1);
                     lj = hi ? s.lin - (unsigned)(nh - 1) * (unsigned)sh : s.lin + (unsigned)(nh - 1) * (unsigned)sh;
-                    aj = label_at<BITS>(lat, lj);
+                    cj = cell_at<BITS>(lat, lj);
+                    aj = (int)(cj & label_mask<BITS>());
                 }
             }
             if (aj < 0) {
@@ -209,29 +230,25 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
                 if (RULE != 0 && !cross) return true;   // a membrane sends the walker back: the rule decides
             }
         }
-        if (cross) {
-            if (aj != s.ai) {
-                rem *= t_ratio[s.ai * NCMAX + aj];
-                s.cur_step = t_step[aj];
-                s.cur_k = t_k[aj];
-                s.ai = aj;
-            }
-            s.lin = lj;
-            const float du = ((up >> hit) & 1u) ? 1.0f : -1.0f;
-            if (hit == 0) s.D0 += du; else if (hit == 1) s.D1 += du; else s.D2 += du;
-        } else {
-            up ^= 1u << hit;
-            if (hit == 0) dl0 = -dl0; else if (hit == 1) dl1 = -dl1; else dl2 = -dl2;
-            h.reflect(hit);
+        if (cross && aj != s.ai) {
+            rem *= t_ratio[s.ai * NCMAX + aj];
+            s.cur_step = t_step[aj];
+            s.cur_k = t_k[aj];
+            s.ai = aj;
         }
+        s.lin = cross ? lj : s.lin;
+        s.cell = cross ? cj : s.cell;
+        const float du = cross ? (dl > 0 ? 1.0f : -1.0f) : 0.0f;
+        const int dn = cross ? dl : -dl;
+        if (hit == 0) { s.D0 += du; dl0 = dn; } else if (hit == 1) { s.D1 += du; dl1 = dn; } else { s.D2 += du; dl2 = dn; }
+        if (!cross) h.reflect(hit);
         // on the face, a whole voxel ahead
         if (hit == 0) d0 = 1.0f; else if (hit == 1) d1 = 1.0f; else d2 = 1.0f;
         if (!(rem > 0.0f)) break;
     }
-    s.o0 = (up & 1u) ? 1.0f - d0 : d0;
-    s.o1 = (up & 2u) ? 1.0f - d1 : d1;
-    s.o2 = (up & 4u) ? 1.0f - d2 : d2;
-    s.cell = cell_at<BITS>(lat, s.lin);
+    s.o0 = dl0 > 0 ? 1.0f - d0 : d0;
+    s.o1 = dl1 > 0 ? 1.0f - d1 : d1;
+    s.o2 = dl2 > 0 ? 1.0f - d2 : d2;
     return false;
 }
 
@@ -240,11 +257,11 @@ __device__ __forceinline__ bool split_step(SplitWalker& s, float v0, float v1, f
 __device__ __forceinline__ void split_direction(float u1, float u2, float& v0, float& v1, float& v2) {
     const float cz = 1.0f - 2.0f * u1;
     const float s2 = u1 * (1.0f - u1);
-    const float sz = 2.0f * s2 * rsqrtf(s2);
-    float sp, cp;
+    const float sz = 2.0f * s2 * rsqrt_approx(s2);
     // azimuth 2 pi (u2 - 1/2): uniform on [-pi, pi), within the hardware
     // sine/cosine's accurate range
-    __sincosf(6.283185307179586f * (u2 - 0.5f), &sp, &cp);
+    const float az = 6.283185307179586f * (u2 - 0.5f);
+    const float sp = sin_approx(az), cp = cos_approx(az);
     v0 = sz * cp; v1 = sz * sp; v2 = cz;
 }
 
