@@ -28,7 +28,11 @@ namespace {
 thread_local std::string g_last_error;
 
 constexpr int kCompatBlock = 128;
-constexpr int kSplitVariantDefault = 0;   // 256 threads, >= 4 blocks per SM (64 registers): fastest measured
+// 128 threads, >= 8 blocks per SM (64 registers; waveforms and membrane rules:
+// 256 x 4, the one built for them).  Small blocks end closer together: 5e4
+// walkers 2.70 ms at 256 x 4, 2.52 at 128 x 8; 2e5 with 90 b-values 16.6 / 16.0;
+// 1e5 and 1e6 walkers within 1 %.
+constexpr int kSplitVariantDefault = 3;
 constexpr int kMaxGrad = 1 << 16;
 constexpr uint64_t kBatchSeedStep = 0x9E3779B97F4A7C15ull;   // seed of batch member k: seed + k * this
 
