@@ -167,17 +167,20 @@ struct rms_device_state {
     int device = -1;
     cudaStream_t own = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
-    DevBuf labels, packed, axons, wavef, tables, rows, slots, sig_slots, vscr, qtab, bvec, grad, gpair, ev_step,
+    DevBuf labels, packed4, packed8, axons, wavef, tables, rows, slots, sig_slots, vscr, qtab, bvec, grad, gpair, ev_step,
         ev_pair, ev_coef, out, out_sig, err, tr_init, tr_vox, tr_ev, tr_pos, adj_g, adj_sums, adj_dwave, adj_ck, adj_ws, adj_blist, adj_bcount, adj_xbin, adj_ajw, adj_wq,
         stage, counts;
     HostPinned h_out, h_axons;
     size_t labels_bytes = 0;
-    bool packed_valid = false;
-    int packed_bits = 0;       // cell width of the packed lattice (4 or 8)
+    // the padded packed lattice in each cell width a launch has asked for
+    bool packed4_valid = false, packed8_valid = false;
+    DevBuf& packed(int bits) { return bits == 4 ? packed4 : packed8; }
+    bool& packed_valid(int bits) { return bits == 4 ? packed4_valid : packed8_valid; }
+    void lattice_changed() { packed4_valid = packed8_valid = false; }
 
     ~rms_device_state() {
         if (device >= 0) cudaSetDevice(device);
-        for (DevBuf* b : {&labels, &packed, &axons, &wavef, &tables, &rows, &slots, &sig_slots, &vscr, &qtab, &bvec, &grad,
+        for (DevBuf* b : {&labels, &packed4, &packed8, &axons, &wavef, &tables, &rows, &slots, &sig_slots, &vscr, &qtab, &bvec, &grad,
                           &gpair, &ev_step, &ev_pair, &ev_coef, &out, &out_sig, &err, &tr_init,
                           &tr_vox, &tr_ev, &tr_pos, &adj_g, &adj_sums, &adj_dwave, &adj_ck, &adj_ws, &adj_blist,
                           &adj_bcount, &adj_xbin, &adj_ajw, &adj_wq, &stage, &counts})
@@ -565,18 +568,16 @@ int prepare_lattice(rms_sim* s, cudaStream_t st, bool split, int bits) {
         RMS_CUDA(d->labels.ensure(s->labels.size()));
         RMS_CUDA(cudaMemcpyAsync(d->labels.p, s->labels.data(), s->labels.size(), cudaMemcpyHostToDevice, st));
         d->labels_bytes = s->labels.size();
-        d->packed_valid = false;
+        d->lattice_changed();
         s->lattice_dirty = false;
     }
-    // packed again when the launch needs another cell width (a batch's widest
-    // Nc decides it for all its members)
-    if (split && (!d->packed_valid || d->packed_bits != bits)) {
-        RMS_CUDA(d->packed.ensure(padded_lattice_bytes(s->n1, s->n2, s->n3, bits)));
+    if (split && !d->packed_valid(bits)) {
+        DevBuf& packed = d->packed(bits);
+        RMS_CUDA(packed.ensure(padded_lattice_bytes(s->n1, s->n2, s->n3, bits)));
         int pe = pack_lattice_padded(d->labels.as<uint8_t>(), s->n1, s->n2, s->n3, bits,
-                                     s->boundary == RMS_BOUNDARY_MIRROR ? 1 : 0, d->packed.as<uint8_t>(), st);
+                                     s->boundary == RMS_BOUNDARY_MIRROR ? 1 : 0, packed.as<uint8_t>(), st);
         if (pe) return cuda_fail((cudaError_t)pe, "label packing");
-        d->packed_valid = true;
-        d->packed_bits = bits;
+        d->packed_valid(bits) = true;
     }
     return RMS_OK;
 }
@@ -587,6 +588,19 @@ int prepare_lattice(rms_sim* s, cudaStream_t st, bool split, int bits) {
 int split_row_sets(int64_t warps, size_t row_sz) {
     const int64_t fit = std::max<int64_t>(1, (int64_t)(((size_t)256 << 20) / (row_sz * sizeof(double))));
     return (int)std::max<int64_t>(1, std::min<int64_t>({warps / 64, 16, fit}));
+}
+
+// Cell width of a split launch.  A byte a cell needs no shifting and masking
+// (five instructions a gather), half a byte keeps a large lattice in the 126 MB
+// L2: bytes for Nc = 8 and for lattices of at most 64 M cells, 48 M with several
+// axons, of which two are walked at a time.  1e6 walkers, walk ms at 4 / 8 bits:
+// 128x128x900 10.3 / 9.9 (2000 steps), 192x192x1536 2.49 / 2.43, 256x256x2048
+// 2.51 / 3.11 (500 steps).
+int launch_cell_bits(const std::vector<LaunchJob>& jobs, int nc_max) {
+    size_t cells = 0;
+    for (const LaunchJob& j : jobs) cells = std::max(cells, padded_lattice_bytes(j.s->n1, j.s->n2, j.s->n3, 8));
+    if (cells <= ((size_t)(jobs.size() == 1 ? 64 : 48) << 20)) return 8;
+    return split_lattice_bits(nc_max);
 }
 
 // Walkers of a tile (one warp's) of a launch over nwalk walkers: 32, and fewer
@@ -705,7 +719,7 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
         tile_w = (int)std::min<int64_t>(32, std::max<int64_t>(tile_w, nwalk / std::max<int64_t>(most, 1) + 1));
         variant = compat_form(s, trace_n > 0, dev_sms, (nwalk + tile_w - 1) / tile_w, row_bytes, per_sm);
     } else {
-        lattice_bits = split_lattice_bits(nc_max);
+        lattice_bits = launch_cell_bits(jobs, nc_max);
         variant = (o && o->variant > 0) ? o->variant - 1 : kSplitVariantDefault;
         if (!split_variant_walks(variant, s->mode, s->rule)) variant = 0;   // waveforms and rules: first variant
         if (variant >= split_variant_count()) return set_error(RMS_ERR_ARG, "variant out of range");
@@ -773,7 +787,7 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
         for (int k = 0; k < naxons; ++k) {
             AxonDesc& x = p.axons[k];
             fill_axon_desc(x, jobs[k].s, jobs[k].w0, jobs[k].w1, tile_begin[k], jobs[k].seed,
-                           jobs[k].s->dev->packed.as<uint8_t>());
+                           jobs[k].s->dev->packed(lattice_bits).as<uint8_t>());
             x.ncopy = split_row_sets(std::min<int64_t>(tile_begin[k + 1] - tile_begin[k], nwarps), row_sz);
             x.row_off = (int64_t)nsets;
             nsets += (size_t)x.ncopy * row_sz;
@@ -1046,7 +1060,7 @@ std::vector<const void*> graph_buffers(const rms_graph* g) {
     std::vector<const void*> v{d->axons.p, d->rows.p, d->slots.p, d->out.p, d->err.p, d->sig_slots.p, d->out_sig.p,
                                d->vscr.p, d->tables.p, d->qtab.p, d->bvec.p, d->grad.p, d->gpair.p,
                                d->ev_step.p, d->ev_pair.p, d->ev_coef.p, d->wavef.p, d->h_out.p, d->h_axons.p};
-    for (const LaunchJob& j : g->jobs) v.push_back(j.s->dev ? j.s->dev->packed.p : nullptr);
+    for (const LaunchJob& j : g->jobs) v.push_back(j.s->dev ? j.s->dev->packed(g->plan.bits).p : nullptr);
     return v;
 }
 
@@ -1085,7 +1099,7 @@ int graph_create(rms_sim* const* sims, int n, const rms_run_opts* o, rms_graph**
 
 int graph_run(rms_graph* g, uint64_t seed) {
     for (const LaunchJob& j : g->jobs)
-        if (j.s->lattice_dirty || !j.s->dev || !j.s->dev->packed_valid || j.s->dev->packed_bits != g->plan.bits)
+        if (j.s->lattice_dirty || !j.s->dev || !j.s->dev->packed_valid(g->plan.bits))
             return set_error(RMS_ERR_STATE, "a simulation of the graph has a new lattice: create the graph again");
     if (graph_buffers(g) != g->buffers)
         return set_error(RMS_ERR_STATE, "the graph's device buffers were reallocated by another run: create the graph again");
@@ -1222,7 +1236,7 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
     if (rc) return rc;
 
     AxonDesc x;
-    fill_axon_desc(x, s, w0, w1, 0, o ? o->seed : 0, d->packed.as<uint8_t>());
+    fill_axon_desc(x, s, w0, w1, 0, o ? o->seed : 0, d->packed(4).as<uint8_t>());
     AdjArgs a{};
     a.lat = x.lat;
     a.n1 = x.n1; a.n2 = x.n2; a.n3 = x.n3; a.s0 = x.s0; a.s1 = x.s1;
@@ -1526,7 +1540,7 @@ int set_lattice_on_device(rms_sim* s, const uint8_t* labels, size_t n) {
     }
     std::swap(d->labels, d->stage);
     d->labels_bytes = n;
-    d->packed_valid = false;
+    d->lattice_changed();
     s->have_lattice = true;
     s->lattice_dirty = false;
     s->host_stale = true;
@@ -1712,7 +1726,7 @@ int rms_sim_set_tube_lattice(rms_sim* s, const double* r2, const double* cx, con
         s->lattice_dirty = false;
         s->host_stale = false;
         d->labels_bytes = nvox;
-        d->packed_valid = false;
+        d->lattice_changed();
         return RMS_OK;
     } catch (const std::exception& ex) {
         return set_error(RMS_ERR_NOMEM, ex.what());

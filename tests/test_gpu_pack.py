@@ -43,3 +43,21 @@ def test_one_label_is_free_diffusion_to_the_walls():
     x2 = o["dx2"][0, [0, 3, 5]] / o["sig0"][0]
     # var(cos^2) = 4/45: standard error of the mean 0.9 / sqrt(4e5) relative, 6 of them
     assert np.abs(x2 / want - 1).max() < 6 * 0.9 / 400000 ** 0.5
+
+
+def test_both_cell_widths_walk_the_same_walkers():
+    """A lattice between the limits for one axon and for several: byte cells in
+    its own launch, half bytes beside a second axon."""
+    from rms_b200 import geometry
+    kw = dict(dt=2e-4, tn=200, npar=20000, res=0.1, diffusivity=[0, 2.0, 1.5], t2=[80, 80, 60], timepoints=10,
+              bval=[], bvec=np.zeros((0, 3)), permeation="kappa", kappa=0.05)
+    big = engine.Sim(shape=(372, 372, 370), **kw)
+    big.set_tube_lattice(*geometry.axon_slices(372, 372, 370, 0.1, 1), inside=1, outside=2)
+    small = engine.Sim(shape=(32, 32, 40), **kw)
+    small.set_tube_lattice(*geometry.axon_slices(32, 32, 40, 0.1, 2), inside=1, outside=2)
+    alone = big.run(seed=5, precision="split").outputs()
+    engine.batch_run([big, small], seed=5, precision="split")
+    both = big.outputs()
+    assert np.array_equal(alone["npar_count"], both["npar_count"])
+    for k in ("sig0", "dx2", "dx4"):
+        np.testing.assert_allclose(both[k], alone[k], rtol=1e-10, atol=1e-12 * np.abs(alone[k]).max())
