@@ -188,9 +188,9 @@ struct LaneArr {
 // the order of the float and FP64 sums.
 constexpr int adj_min_blocks(bool jac, int form) { return form == 1 ? 6 : (form == 2 ? 5 : (jac ? 1 : 5)); }
 
-template <bool JAC, int FORM>
+template <bool JAC, int FORM, int BITS>
 __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_kernel(const __grid_constant__ AdjArgs a) {
-    constexpr int NC = kAdjNc, BITS = 4, NW = kAdjWaves;
+    constexpr int NC = kAdjNc, NW = kAdjWaves;
     constexpr int kTab = 2 * NC + 2 * NC * NC;
     __shared__ float s_tab[kTab];
     // per lane (LaneArr): phi; dphi but in the weighted FORM 2; and a_jw (FORM 0)
@@ -771,29 +771,33 @@ int launch_adjoint_dwave(const AdjArgs& a, int sms, void* stream) {
     return (int)cudaGetLastError();
 }
 
-template <bool JAC>
-static int launch_form(const AdjArgs& a, int form, int grid, cudaStream_t st) {
-    if (form == 0) adjoint_kernel<JAC, 0><<<grid, kAdjBlock, 0, st>>>(a);
-    else if (form == 1) adjoint_kernel<JAC, 1><<<grid, kAdjBlock, 0, st>>>(a);
-    else adjoint_kernel<JAC, 2><<<grid, kAdjBlock, 0, st>>>(a);
-    return (int)cudaGetLastError();
+// The kernel of a form and cell width (rms_api.cpp takes byte cells where they
+// fit L2, as the split walk does).
+template <class F>
+static auto by_form(bool jac, int form, int bits, F&& f) {
+    auto width = [&]<bool J, int FM>() {
+        return bits == 4 ? f(adjoint_kernel<J, FM, 4>) : f(adjoint_kernel<J, FM, 8>);
+    };
+    auto forms = [&]<bool J>() {
+        return form == 0 ? width.template operator()<J, 0>()
+                         : (form == 1 ? width.template operator()<J, 1>() : width.template operator()<J, 2>());
+    };
+    return jac ? forms.template operator()<true>() : forms.template operator()<false>();
 }
 
-template <bool JAC>
-static int blocks_form(int form) {
-    int n = 0;
-    const cudaError_t e =
-        form == 0   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_kernel<JAC, 0>, kAdjBlock, 0)
-        : form == 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_kernel<JAC, 1>, kAdjBlock, 0)
-                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_kernel<JAC, 2>, kAdjBlock, 0);
-    return e == cudaSuccess ? n : -1;
+int launch_adjoint(const AdjArgs& a, int bits, bool jac, int form, int grid, void* stream) {
+    return by_form(jac, form, bits, [&](auto* kernel) {
+        kernel<<<grid, kAdjBlock, 0, (cudaStream_t)stream>>>(a);
+        return (int)cudaGetLastError();
+    });
 }
 
-int launch_adjoint(const AdjArgs& a, bool jac, int form, int grid, void* stream) {
-    return jac ? launch_form<true>(a, form, grid, (cudaStream_t)stream)
-               : launch_form<false>(a, form, grid, (cudaStream_t)stream);
+int adjoint_blocks_per_sm(int bits, bool jac, int form) {
+    return by_form(jac, form, bits, [&](auto* kernel) {
+        int n = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kAdjBlock, 0);
+        return e == cudaSuccess ? n : -1;
+    });
 }
-
-int adjoint_blocks_per_sm(bool jac, int form) { return jac ? blocks_form<true>(form) : blocks_form<false>(form); }
 
 }  // namespace rms

@@ -1232,11 +1232,12 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
     rms_device_state* d = s->dev;
     RMS_CUDA(cudaSetDevice(device));
     cudaStream_t st = (o && o->stream) ? (cudaStream_t)o->stream : d->own;
-    rc = prepare_lattice(s, st, true, 4);
+    const int bits = launch_cell_bits({LaunchJob{s, w0, w1, 0}}, s->nc);
+    rc = prepare_lattice(s, st, true, bits);
     if (rc) return rc;
 
     AxonDesc x;
-    fill_axon_desc(x, s, w0, w1, 0, o ? o->seed : 0, d->packed(4).as<uint8_t>());
+    fill_axon_desc(x, s, w0, w1, 0, o ? o->seed : 0, d->packed(bits).as<uint8_t>());
     AdjArgs a{};
     a.lat = x.lat;
     a.n1 = x.n1; a.n2 = x.n2; a.n3 = x.n3; a.s0 = x.s0; a.s1 = x.s1;
@@ -1303,7 +1304,7 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
     RMS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int64_t wpb = kAdjBlock / 32;
     auto grid_for = [&](int form, int64_t tiles, int& grid) -> int {
-        const int per_sm = adjoint_blocks_per_sm(jac != nullptr, form);
+        const int per_sm = adjoint_blocks_per_sm(bits, jac != nullptr, form);
         if (per_sm <= 0) return set_error(RMS_ERR_CUDA, "occupancy query failed (kernel image missing for this GPU?)");
         grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * per_sm, (tiles + wpb - 1) / wpb));
         return RMS_OK;
@@ -1376,7 +1377,7 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
         int grid = 0;
         rc = grid_for(0, a.ntiles, grid);
         if (rc) return rc;
-        const int e = launch_adjoint(a, jac != nullptr, 0, grid, st);
+        const int e = launch_adjoint(a, bits, jac != nullptr, 0, grid, st);
         if (e) return cuda_fail((cudaError_t)e, "adjoint kernel launch");
     } else {
         a.ck_every = (int)ck_every;
@@ -1396,7 +1397,7 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
             int grid = 0;
             rc = grid_for(1, a.ntiles, grid);
             if (rc) return rc;
-            int e = launch_adjoint(a, jac != nullptr, 1, grid, st);
+            int e = launch_adjoint(a, bits, jac != nullptr, 1, grid, st);
             if (e) return cuda_fail((cudaError_t)e, "adjoint kernel launch (pass 1)");
             if (!jac) {
                 e = launch_adjoint_dwave(a, sms, st);
@@ -1407,7 +1408,7 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
                 a.ntiles = a.nwalk / 32 + nbk;
                 rc = grid_for(2, a.ntiles, grid);
                 if (rc) return rc;
-                e = launch_adjoint(a, jac != nullptr, 2, grid, st);
+                e = launch_adjoint(a, bits, jac != nullptr, 2, grid, st);
                 if (e) return cuda_fail((cudaError_t)e, "adjoint kernel launch (forced walks)");
             }
         }

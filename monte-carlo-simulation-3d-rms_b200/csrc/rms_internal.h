@@ -160,7 +160,7 @@ constexpr int kAdjSums = kAdjSumForce + 1;
 constexpr int kJacE = 0, kJacTR = 2 * kAdjWaves, kJacF = 4 * kAdjWaves, kJacLT = 6 * kAdjWaves;
 constexpr int kJacSums = kJacLT + 2 * kAdjWaves * kAdjNc;
 struct AdjArgs {
-    const uint8_t* lat;          // padded 4-bit lattice with free-flight flags
+    const uint8_t* lat;          // padded lattice with free-flight flags
     int n1, n2, n3, s0, s1;
     int64_t walker_begin, walker_end, ntiles;
     uint64_t seed;
@@ -194,9 +194,9 @@ struct AdjArgs {
 // and the buckets of the forced walks; 2: the forced walks, grouped by resume
 // step.  launch_adjoint_dwave: dL/dwave from form 1's X_wb and a_jw.
 constexpr int kAdjCkWords = 23 + kAdjWaves, kAdjWsWords = 3 + kAdjWaves, kAdjCkMax = 16;
-int launch_adjoint(const AdjArgs& a, bool jac, int form, int grid, void* stream);
+int launch_adjoint(const AdjArgs& a, int bits, bool jac, int form, int grid, void* stream);
 int launch_adjoint_dwave(const AdjArgs& a, int sms, void* stream);
-int adjoint_blocks_per_sm(bool jac, int form);
+int adjoint_blocks_per_sm(int bits, bool jac, int form);   // bits: a.lat's cell width
 constexpr int kAdjBlock = 128;
 
 // Multi-waveform phase contraction (rms_contract.cu): out[j] = (sum_w cos phi,
