@@ -23,6 +23,7 @@
 
 #include "philox.cuh"
 #include "rms_internal.h"
+#include "warp_reduce.cuh"
 
 namespace rms {
 namespace {
@@ -48,11 +49,12 @@ __device__ __forceinline__ double face_time(double d, double v) {
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
 // Dev. 34, 1990, theorem 8.3) -- the division's own result, without forming the
 // reciprocal of the same b again for every a.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-    double q = __dmul_rn(a, y);
+__device__ __forceinline__ double div_by(double a, double b, double y, double q) {   // q: a * y
     q = __fma_rn(__fma_rn(-q, b, a), y, q);
     return __fma_rn(__fma_rn(-q, b, a), y, q);
 }
+
+__device__ __forceinline__ double div_by(double a, double b, double y) { return div_by(a, b, y, __dmul_rn(a, y)); }
 
 // Records in batches of kRec, as the split walk takes them
 // (rms_walk_split.cu): every lane stages its walker's displacement and T2
@@ -111,41 +113,63 @@ __device__ __noinline__ void add_moments(double* st, double* row, int nvals, int
     }
 }
 
-// narrow-pulse signals of a batch (main.cu:374-378)
+// Narrow-pulse signals of a batch (main.cu:374-378).  Lanes beyond the b-values
+// of a group of 32 take a share of the walkers (signal_lanes).
 __device__ __noinline__ void add_signals(const double* st, const double* __restrict__ qtab,
                                          const double* __restrict__ bvec, int nb, double* row, int nvals, int nrec,
                                          int nw, bool first, int lane) {
     __syncwarp();
-    for (int jb = lane; jb < nb; jb += 32) {
-        const double bx = __ldg(bvec + jb * 3), by = __ldg(bvec + jb * 3 + 1), bz = __ldg(bvec + jb * 3 + 2);
+    auto group = [&](int jb, bool in, int first_w, int step, auto&& total) {
+        const double bx = in ? __ldg(bvec + jb * 3) : 0.0, by = in ? __ldg(bvec + jb * 3 + 1) : 0.0,
+                     bz = in ? __ldg(bvec + jb * 3 + 2) : 0.0;
         for (int r = 0; r < nrec; ++r) {
-            const double q = __ldg(qtab + (size_t)r * nb + jb);
+            const double q = in ? __ldg(qtab + (size_t)r * nb + jb) : 0.0;
             const double* v = st + r * kStageRow;
             double s = 0.0;
 #pragma unroll 2
-            for (int w = 0; w < nw; ++w) s += v[96 + w] * cos(q * (v[w] * bx + v[32 + w] * by + v[64 + w] * bz));
-            put(row + (size_t)r * nvals + jb, s, first);
+            for (int w = first_w; w < nw; w += step)
+                s += v[96 + w] * cos(q * (v[w] * bx + v[32 + w] * by + v[64 + w] * bz));
+            total(row + (size_t)r * nvals + jb, s);
         }
+    };
+    int base = 0;
+    // a lane to a b-value, while more than half the lanes have one
+    for (; nb - base > 16 || (base < nb && nw == 1); base += 32) {
+        const int jb = base + lane;
+        if (jb < nb) group(jb, true, 0, 1, [&](double* p, double s) { put(p, s, first); });
+    }
+    if (base < nb) {
+        const SignalLanes l = signal_lanes(lane, nb - base, nw);
+        const int jb = base + l.item;
+        const bool in = jb < nb;
+        group(jb, in, l.share, l.shares, [&](double* p, double s) {
+            s = share_sum(s, l);
+            if (in && l.share == 0) put(p, s, first);
+        });
     }
 }
 
-// Final T2-weighted PGSE signal of the tile (main_PGSE.cu:348-357), lane j one
-// gradient: phase_j = |g| (g_hat . V) dt with the walkers' window sums V in vscr
-// ([pair * 3 + axis][thread], thread t0 + w).
+// Final T2-weighted PGSE signal of the tile (main_PGSE.cu:348-357), a lane (or
+// several) to a gradient: phase_j = |g| (g_hat . V) dt with the walkers' window
+// sums V in vscr ([pair * 3 + axis][thread], thread t0 + w).
 __device__ __noinline__ void add_pgse(const WalkArgs& a, int nthr, int t0, double s0, int nw, double* sig, bool first,
                                       int lane) {
     __syncwarp();
     for (int base = 0; base < a.ngrad; base += 32) {
-        const int j = min(base + lane, a.ngrad - 1);
+        const SignalLanes l = signal_lanes(lane, min(32, a.ngrad - base), nw);
+        const int j = min(base + l.item, a.ngrad - 1);
         const double* g = a.grad + 6 * j;
         const double* vv = a.vscr + (size_t)(a.gpair[j] * 3) * nthr + t0;
         const double g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5];
         double s = 0.0;
-        for (int w = 0; w < nw; ++w) {
+        for (int k = 0; k < nw; k += l.shares) {
+            const int w = min(k + l.share, nw - 1);
             const double phase = g2 * (vv[w] * g3 + vv[nthr + w] * g4 + vv[2 * (size_t)nthr + w] * g5) * a.dt;
-            s += __shfl_sync(0xffffffffu, s0, w) * cos(phase);
+            const double sw = __shfl_sync(0xffffffffu, s0, w);
+            s += (k + l.share < nw ? sw : 0.0) * cos(phase);
         }
-        if (base + lane < a.ngrad) put(sig + j, s, first);
+        s = share_sum(s, l);
+        if (base + l.item < a.ngrad && l.share == 0) put(sig + j, s, first);
     }
 }
 
@@ -268,21 +292,23 @@ __global__ void __launch_bounds__(kBlock, MINB) walk_compat_kernel(const __grid_
                     const double d0 = f0 - xt0, d1 = f1 - xt1, d2 = f2 - xt2;
                     const double u0 = d0 * y0, u1 = d1 * y1, u2 = d2 * y2;
                     const bool b1 = u1 < u0;
-                    const double lo = b1 ? u1 : u0, hi = b1 ? u0 : u1;
+                    const double lo = b1 ? u1 : u0;
                     const bool b2 = u2 < lo;
-                    double tmin = b2 ? u2 : lo;
-                    const double next = b2 ? lo : (u2 < hi ? u2 : hi);
+                    const double u = b2 ? u2 : lo;
+                    double tmin = u;
                     int hit = b2 ? 2 : (b1 ? 1 : 0);
                     const double st_ = s_step[ai];                  // main.cu:231-244
                     const double reach = fstep * st_;
                     bool ends = reach * kNear < tmin;
                     if (!ends) {
-                        tmin = tmin > 0.0 ? tmin : 0.0;
-                        if (reach > tmin * kNear && next > tmin * kNear) {
+                        // (a face already passed by rounding is reached at once)
+                        const double th = tmin > 0.0 ? tmin * kNear : 0.0;
+                        const int near = (int)(u0 <= th) + (int)(u1 <= th) + (int)(u2 <= th);
+                        if (reach > th && near == 1) {
                             const double d = hit == 0 ? d0 : (hit == 1 ? d1 : d2);
                             const double v = hit == 0 ? v0 : (hit == 1 ? v1 : v2);
                             const double y = hit == 0 ? y0 : (hit == 1 ? y1 : y2);
-                            const double q = div_by(d, v, y);
+                            const double q = div_by(d, v, y, u);
                             tmin = (0.0 < q) ? q : 0.0;
                         } else {
                             // too close to call: the exact quotients, lowest axis on ties

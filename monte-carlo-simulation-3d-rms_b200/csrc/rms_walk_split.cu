@@ -272,18 +272,16 @@ __device__ __noinline__ void add_moments(const float* st, const unsigned* msk, d
     }
 }
 
-// The batch's narrow-pulse signals: lane j holds b-value base + j and adds
-// s0 cos(q n.dx) over the tile's walkers, read as broadcasts from the staged
-// rows -- one cosine, one conversion and one FP64 add per walker and b-value.
+// The batch's narrow-pulse signals: a lane (or several, signal_lanes) holds one
+// b-value and adds s0 cos(q n.dx) over the tile's walkers, read as broadcasts
+// from the staged rows -- one cosine, one conversion and one FP64 add per walker and b-value.
 // One b-value at a time over the 32 lanes took 10 shuffles and 5 FP64 adds more.
 template <bool ONE>
 __device__ __noinline__ void add_signals(const float* st, const double* __restrict__ qtab,
                                          const double* __restrict__ bvec, int nb, double* dst, int stride, int nrec,
                                          int nw, int lane) {
     __syncwarp();
-    for (int base = 0; base < nb; base += 32) {
-        const int jb = base + lane;
-        const bool in = jb < nb;
+    auto group = [&](int jb, bool in, int first_w, int step, auto&& total) {
         const float bx = in ? (float)__ldg(bvec + jb * 3) : 0.0f, by = in ? (float)__ldg(bvec + jb * 3 + 1) : 0.0f,
                     bz = in ? (float)__ldg(bvec + jb * 3 + 2) : 0.0f;
         for (int r = 0; r < nrec; ++r) {
@@ -295,15 +293,30 @@ __device__ __noinline__ void add_signals(const float* st, const double* __restri
             };
             double s = 0.0;
 #pragma unroll 1
-            for (int w = 0; w < nw; w += 4) {
+            for (int w = first_w; w < nw; w += step) {
                 // past the tile's walkers the weights are zero
                 const float4 X = *reinterpret_cast<const float4*>(v + w), Y = *reinterpret_cast<const float4*>(v + 32 + w),
                              Z = *reinterpret_cast<const float4*>(v + 64 + w), S = *reinterpret_cast<const float4*>(v + 96 + w);
                 s += (cosine(X.x, Y.x, Z.x, S.x) + cosine(X.y, Y.y, Z.y, S.y)) +
                      (cosine(X.z, Y.z, Z.z, S.z) + cosine(X.w, Y.w, Z.w, S.w));
             }
-            if (in) add_out<ONE>(dst + (size_t)r * stride + jb, s);
+            total(dst + (size_t)r * stride + jb, s);
         }
+    };
+    int base = 0;
+    // a lane to a b-value, while more than half the lanes have one
+    for (; nb - base > 16 || (base < nb && nw <= 4); base += 32) {
+        const int jb = base + lane;
+        if (jb < nb) group(jb, true, 0, 4, [&](double* p, double s) { add_out<ONE>(p, s); });
+    }
+    if (base < nb) {
+        const SignalLanes l = signal_lanes(lane, nb - base, (nw + 3) / 4);   // (walkers go by fours)
+        const int jb = base + l.item;
+        const bool in = jb < nb;
+        group(jb, in, 4 * l.share, 4 * l.shares, [&](double* p, double s) {
+            s = share_sum(s, l);
+            if (in && l.share == 0) add_out<ONE>(p, s);
+        });
     }
 }
 
@@ -329,6 +342,33 @@ __device__ __forceinline__ void unpark_walker(const volatile uint32_t* p, SplitW
     w.w32 = __uint_as_float(p[14]);
     perm.q1 = p[15]; perm.q2 = p[16]; perm.q3 = p[17];
     q0 = __uint_as_float(p[18]); q1 = __uint_as_float(p[19]); q2 = __uint_as_float(p[20]); q3 = __uint_as_float(p[21]);
+}
+
+// Final T2-weighted PGSE signal of a tile, a lane (or several) to a gradient:
+// phase_j = |g| (g_hat . V) res dt with the walkers' window sums V in vscr
+// ([pair * 3 + axis][thread], thread t0 + w).  One gradient at a time over the
+// 32 walkers took 10 shuffles and 5 FP64 adds more, and a warp's 32 lanes for
+// however few walkers its tile has.
+template <bool ONE>
+__device__ __forceinline__ void add_pgse(const WalkArgs& a, int nthr, int t0, double s0, int nw, double* sig, int lane) {
+    __syncwarp();
+    const double scale = a.res * a.dt;
+    for (int base = 0; base < a.ngrad; base += 32) {
+        const SignalLanes l = signal_lanes(lane, min(32, a.ngrad - base), nw);
+        const int j = min(base + l.item, a.ngrad - 1);
+        const double* g = a.grad + 6 * j;
+        const double* vv = a.vscr + (size_t)(a.gpair[j] * 3) * nthr + t0;
+        const double g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5];
+        double s = 0.0;
+        for (int k = 0; k < nw; k += l.shares) {
+            const int w = min(k + l.share, nw - 1);
+            const double phase = g2 * (vv[w] * g3 + vv[nthr + w] * g4 + vv[2 * (size_t)nthr + w] * g5) * scale;
+            const double sw = __shfl_sync(0xffffffffu, s0, w);
+            s += (k + l.share < nw ? sw : 0.0) * cos(phase);
+        }
+        s = share_sum(s, l);
+        if (base + l.item < a.ngrad && l.share == 0) add_out<ONE>(sig + j, s);
+    }
 }
 
 // ONE: the no-allocation walk's form -- one axon, whose scalars are read from
@@ -583,23 +623,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
             if (wave) {
                 wave_final<ONE>(a.vscr + gtid, nthr, a.nwave, active ? exp(-(w64 + (double)wk.w32)) : 0.0, sig_slot, lane);
             } else {
-                // final T2-weighted signal: phase_j = |g| (g_hat . V) res dt
-                const double s0 = active ? exp(-(w64 + (double)wk.w32)) : 0.0;
-                const double scale = a.res * a.dt;
-                for (int base = 0; base < a.ngrad; base += 32) {
-                    double mine = 0.0;
-                    const int cnt = min(32, a.ngrad - base);
-                    for (int k = 0; k < cnt; ++k) {
-                        const int jg = base + k;
-                        const double* vv = a.vscr + (size_t)(a.gpair[jg] * 3) * nthr + gtid;
-                        const double* g = a.grad + 6 * jg;
-                        const double phase =
-                            g[2] * (vv[0] * g[3] + vv[nthr] * g[4] + vv[2 * (size_t)nthr] * g[5]) * scale;
-                        const double r = warp_sum(s0 * cos(phase));
-                        if (lane == k) mine = r;
-                    }
-                    if (lane < cnt) add_out<ONE>(sig_slot + base + lane, mine);
-                }
+                add_pgse<ONE>(a, nthr, gtid - lane, active ? exp(-(w64 + (double)wk.w32)) : 0.0, tile_w, sig_slot, lane);
             }
         }
     }

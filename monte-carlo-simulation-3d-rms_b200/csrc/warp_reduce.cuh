@@ -26,38 +26,25 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// Reduce-scatter of 32 values held by every lane: on return lane l holds the
-// warp-wide sum of v[l].  Each halving level exchanges half of the remaining
-// values (16 + 8 + 4 + 2 + 1 = 31 shuffles instead of 32 x 5).
-__device__ __forceinline__ double warp_reduce_scatter32(double (&v)[32], int lane) {
-#pragma unroll
-    for (int half = 16; half > 0; half >>= 1) {
-        const bool upper = (lane & half) != 0;
-#pragma unroll
-        for (int k = 0; k < half; ++k) {
-            const double send = upper ? v[k] : v[k + half];
-            const double keep = upper ? v[k + half] : v[k];
-            v[k] = keep + __shfl_xor_sync(kFullMask, send, half);
-        }
+// The lanes of a warp over `items` (at most 32: b-values, gradients) and a
+// tile's nw walkers: lane -> (item, share of the walkers), with as many shares
+// as the items leave lanes for -- twelve b-values over 32 walkers are two shares
+// of 16, not 20 idle lanes.
+struct SignalLanes {
+    int item, share, shares, per;   // per: lanes of a share, a power of two
+};
+__device__ __forceinline__ SignalLanes signal_lanes(int lane, int items, int nw) {
+    int per = 32, shares = 1;
+    while (per / 2 >= items && 2 * shares <= nw) {
+        per >>= 1;
+        shares <<= 1;
     }
-    return v[0];
+    return SignalLanes{lane & (per - 1), lane / per, shares, per};
 }
-
-// Reduce-scatter of 16 values: on return lanes l and l ^ 16 both hold the
-// warp-wide sum of v[l & 15] (8 + 4 + 2 + 1 halving shuffles, then one
-// butterfly across the half-warps).  Half the registers of the 32-value form.
-__device__ __forceinline__ double warp_reduce_scatter16(double (&v)[16], int lane) {
-#pragma unroll
-    for (int half = 8; half > 0; half >>= 1) {
-        const bool upper = (lane & half) != 0;
-#pragma unroll
-        for (int k = 0; k < half; ++k) {
-            const double send = upper ? v[k] : v[k + half];
-            const double keep = upper ? v[k + half] : v[k];
-            v[k] = keep + __shfl_xor_sync(kFullMask, send, half);
-        }
-    }
-    return v[0] + __shfl_xor_sync(kFullMask, v[0], 16);
+// Sum over an item's shares (every lane of the warp calls it).
+__device__ __forceinline__ double share_sum(double s, const SignalLanes& l) {
+    for (int off = l.per; off < 32; off <<= 1) s += __shfl_xor_sync(kFullMask, s, off);
+    return s;
 }
 
 }  // namespace rms

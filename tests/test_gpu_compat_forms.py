@@ -80,3 +80,18 @@ def test_pgse_gradients_per_lane(ng):
                        timepoints=10, td=td, grad=g)
     want = pyoracle.run_oracle(job, nthreads=8)
     assert_fp64_close(got["sig"], want["sig"], 1e-9, "sig")
+
+
+@pytest.mark.parametrize("precision", ["compat", "split"])
+@pytest.mark.parametrize("npar", [3, 5000, 100_000])
+def test_b_values_shared_between_lanes(npar, precision):
+    """Lanes beyond the b-values of a group share its walkers: each b-value's
+    signal from tables of 1 to 49 of them, which split the lanes in every way,
+    equals its signal from a table of its own (FP64 sums in another order)."""
+    b, v = table(49, seed=1)
+    lab = lattice()
+    kw = dict(dt=2e-4, tn=9, npar=npar, res=0.1, diffusivity=D, t2=T2, timepoints=9)
+    full = engine.Sim(lab, bval=b, bvec=v, **kw).run(seed=6, precision=precision).outputs()["sigre"]
+    for n in (1, 2, 3, 8, 9, 16, 17, 33, 48):
+        got = engine.Sim(lab, bval=b[:n], bvec=v[:n], **kw).run(seed=6, precision=precision).outputs()["sigre"]
+        assert np.abs(got - full[:, :n]).max() <= 1e-12 * npar, n
