@@ -48,6 +48,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "../../include/rms.h"
@@ -95,48 +96,68 @@ __device__ __forceinline__ void sincos_reduced(float phi, float* s, float* c) {
 constexpr int kF32Tile = 128;   // waveforms and walkers per block
 constexpr int kF32Kc = 16;
 
-__global__ void __launch_bounds__(256) contract_f32_kernel(const float* __restrict__ pos, int64_t nwalk, int K,
-                                                           const float* __restrict__ wave, int nwave,
-                                                           int n_mtiles, double* __restrict__ out) {
-    __shared__ float As[kF32Kc][kF32Tile];   // waveforms, [k][m]
-    __shared__ float Bs[kF32Kc][kF32Tile];   // walkers, [k][n]
+// A thread holds 8 waveforms (ty + 16 i) x 8 walkers (tx + 16 j), the walkers of
+// two j side by side for the paired FMA (two products an instruction, each
+// rounded as its own fmaf, k ascending).  Bound by FP32 issue: 32 paired FMAs to
+// 8 shared loads per k.  The next 16 k are on their way from memory while these
+// are multiplied.  300000 walkers x 768 x 1024: 17.6
+// ms with single FMAs, eight scalar loads a side and a barrier on each side of
+// the products, 11.8 now (40 TFLOP/s).
+__global__ void __launch_bounds__(256, 2) contract_f32_kernel(const float* __restrict__ pos, int64_t nwalk, int K,
+                                                              const float* __restrict__ wave, int nwave,
+                                                              int n_mtiles, double* __restrict__ out) {
+    // waveforms [k][m] and walkers [k][n]; 4 floats of padding put the 16 k of a
+    // row, which one half-warp stores, on 16 banks
+    __shared__ __align__(16) float As[2][kF32Kc][kF32Tile + 4], Bs[2][kF32Kc][kF32Tile + 4];
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
     const int mt = (int)(blockIdx.x % n_mtiles);
     const int64_t wt = blockIdx.x / n_mtiles;
     const int m0 = mt * kF32Tile;
     const int64_t n0 = wt * kF32Tile;
+    float2 acc2[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc2[i][j] = make_float2(0.0f, 0.0f);
+    const int lk = tid & 15, lrow = tid >> 4;   // 16 consecutive threads read one row's 16 k
+    float an[8], bn[8];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int row = lrow + 16 * r, m = m0 + row;
+            const int64_t n = n0 + row;
+            an[r] = (m < nwave && k0 + lk < K) ? __ldg(wave + (size_t)m * K + k0 + lk) : 0.0f;
+            bn[r] = (n < nwalk && k0 + lk < K) ? __ldg(pos + (size_t)n * K + k0 + lk) : 0.0f;
+        }
+    };
+    fetch(0);
+    for (int k0 = 0, st = 0; k0 < K; k0 += kF32Kc, st ^= 1) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            As[st][lk][lrow + 16 * r] = an[r];
+            Bs[st][lk][2 * lrow + (r & 1) + 32 * (r >> 1)] = bn[r];   // walkers lrow + 16 r, pairs of r side by side
+        }
+        __syncthreads();   // (a buffer is written again two rounds later, past the next barrier)
+        if (k0 + kF32Kc < K) fetch(k0 + kF32Kc);
+#pragma unroll
+        for (int k = 0; k < kF32Kc; ++k) {
+            float2 b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float2*>(&Bs[st][k][2 * tx + 32 * j]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float a = As[st][k][ty + 16 * i];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc2[i][j] = __ffma2_rn(make_float2(a, a), b[j], acc2[i][j]);
+            }
+        }
+    }
     float acc[8][8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-
-    for (int k0 = 0; k0 < K; k0 += kF32Kc) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int e = tid + 256 * r;         // 0 .. 2047
-            const int k = e & 15, row = e >> 4;  // 16 consecutive threads read one row's 16 k
-            const int m = m0 + row;
-            const int64_t n = n0 + row;
-            As[k][row] = (m < nwave && k0 + k < K) ? __ldg(wave + (size_t)m * K + k0 + k) : 0.0f;
-            Bs[k][row] = (n < nwalk && k0 + k < K) ? __ldg(pos + (size_t)n * K + k0 + k) : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kF32Kc; ++k) {
-            float a[8], b[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = As[k][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) b[j] = Bs[k][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
+        for (int j = 0; j < 4; ++j) { acc[i][2 * j] = acc2[i][j].x; acc[i][2 * j + 1] = acc2[i][j].y; }
     // epilogue: per waveform row, cosine and sine sums over this block's walkers
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -167,21 +188,24 @@ __global__ void __launch_bounds__(256) contract_f32_kernel(const float* __restri
 // tensor-core method
 
 constexpr int kKc = 64;                         // k per pipeline chunk: one 128-byte BF16 row
-constexpr int kTileN = 256;                     // walkers per tile (MMA N)
+// Walkers per tile (MMA N): 256, or 128 or 64 where 256 would leave SMs without
+// a unit (contract_phases): a unit's MMAs, conversions and epilogue all scale
+// with it, and 4763 walkers are 19 units of 256 but 75 of 64.
+constexpr int kTileNMax = 256;
 constexpr int kTileM = 128;                     // waveforms per tile (MMA M)
 constexpr int kBStages = 2;                     // converted position chunks
 constexpr int kGStages = 3;                     // waveform chunks of one tile (a copy is issued once an MMA frees one)
-constexpr uint32_t kXbBytes = kTileN * kKc * 2;         // one BF16 part: 32768
+template <int TN> constexpr uint32_t kXbBytes = TN * kKc * 2;        // one BF16 part: 32768 at TN = 256
 constexpr uint32_t kGBytes = kTileM * kKc * 2;          // one BF16 part: 16384
 constexpr uint32_t kOffXb = 0;
-constexpr uint32_t kOffG = kOffXb + kBStages * 2 * kXbBytes;           // 131072
+constexpr uint32_t kOffG = kOffXb + kBStages * 2 * kXbBytes<kTileNMax>;           // 131072
 constexpr uint32_t kOffBar = kOffG + kGStages * 2 * kGBytes;           // 229376
 constexpr uint32_t kSmemUsed = kOffBar + 256;
 constexpr uint32_t kSmemBytes = kSmemUsed + 1024;                      // + alignment slack
 constexpr int kConvThreads = 256;               // warps 0-7
 constexpr int kWarpEpi = 8, kWarpG = 12, kWarpMma = 13;
 constexpr int kTcThreads = 448;
-constexpr uint32_t kTmemCols = 512;
+template <int TN> constexpr uint32_t kTmemCols = 2 * TN;   // two accumulators of TN columns
 // K-major operands, 128-byte swizzle: row r of a part holds its 64 BF16 k
 // values in 128 bytes, 16-byte chunk c stored at chunk c ^ (r % 8); 8-row
 // groups 1024 B apart (SBO).  An MMA's K = 16 step starts 32 B further in.
@@ -190,9 +214,10 @@ __host__ __device__ constexpr uint32_t sw128_offset(int row, int chunk) {
     return (uint32_t)(row >> 3) * kSbo + (uint32_t)(row & 7) * 128 + (uint32_t)((chunk ^ (row & 7)) << 4);
 }
 // kind::f16 instruction descriptor: D FP32 (bits 4-5 = 1), A and B BF16
-// (bits 7-9, 10-12 = 1), both K-major, N = 256 (bits 17-22: N >> 3),
+// (bits 7-9, 10-12 = 1), both K-major, N = TN (bits 17-22: N >> 3),
 // M = 128 (bits 24-28: M >> 4)
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileN >> 3) << 17) |
+template <int TN>
+constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) |
                             ((uint32_t)(kTileM >> 4) << 24);
 
 // barrier indices (8 bytes each at kOffBar)
@@ -272,12 +297,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(kSbo >> 4) << 32) | (1ull << 46) |
            (2ull << 61);
 }
+template <int TN>
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(kIdesc<TN>), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -308,9 +334,13 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
 
 // Waveforms [nwave][K] FP32 -> per (waveform tile, k chunk) 32 KB blocks:
 // BF16 hi part then lo part, each 128 rows x 64 k, 128-byte swizzle; rows
-// past nwave and k past K are zero.
+// past nwave and k past K are zero.  The error word and the sums start here at
+// zero too (two launches less in front of a small contraction).
 __global__ void pack_waves_kernel(const float* __restrict__ wave, int nwave, int K, int nk, int n_mtiles,
-                                  uint8_t* __restrict__ gpack) {
+                                  uint8_t* __restrict__ gpack, int* err, double* __restrict__ out) {
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid == 0) *err = 0;
+    for (int64_t i = tid; i < 2 * (int64_t)nwave; i += (int64_t)gridDim.x * blockDim.x) out[i] = 0.0;
     const int64_t items = (int64_t)n_mtiles * kTileM * nk * (kKc / 8);   // one item: 8 k of one row
     for (int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; it < items;
          it += (int64_t)gridDim.x * blockDim.x) {
@@ -335,9 +365,13 @@ __global__ void pack_waves_kernel(const float* __restrict__ wave, int nwave, int
     }
 }
 
+template <int TN, bool PAIRS>
 __global__ void __launch_bounds__(kTcThreads, 1)
     contract_tc_kernel(const float* __restrict__ pos, int K, const uint8_t* __restrict__ gpack, int64_t nwalk,
                        int nwave, int nk, int n_mpairs, int64_t nunits, double* __restrict__ out, int* err) {
+    // waveform tiles of a pair: the last pair's second tile may hold no waveform
+    // (PAIRS: never, and no role looks; 1 % of a full contraction)
+    auto tiles = [&](int mp) { return PAIRS || (2 * mp + 1) * kTileM < nwave ? 2 : 1; };
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
@@ -365,7 +399,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
     if (warp == kWarpMma) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(sbase + kOffTmemSlot), "r"(kTmemCols)
+                     ::"r"(sbase + kOffTmemSlot), "r"(kTmemCols<TN>)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -381,9 +415,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             int64_t j = 0;
             bool ok = true;
             for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
-                const int mp = (int)(u % n_mpairs);
+                const int mp = (int)(u % n_mpairs), na = tiles(mp);
                 for (int kc = 0; kc < nk && ok; ++kc) {
-                    for (int a = 0; a < 2; ++a, ++j) {
+                    for (int a = 0; a < na; ++a, ++j) {
                         const int s = (int)(j % kGStages);
                         if (!(ok = mbar_wait(bar(kBarGEmpty + s), (uint32_t)((j / kGStages) & 1) ^ 1u, abort_flag, err,
                                              true)))
@@ -409,12 +443,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const int ct = threadIdx.x;   // 0 .. kConvThreads - 1
         const int g = (ct >> 3) & 3;
         const int rw = ((ct >> 5) << 3) + (ct & 7);   // row within a 64-row slab
-        float4 cur[8], nxt[8];
-        auto load = [&](int64_t uu, int kk, int hh, float4(&v)[8]) {
-            const int64_t w0 = (uu / n_mpairs) * kTileN;
+        constexpr int kIt = TN / 64;   // 64-row slabs of a chunk
+        float4 cur[2 * kIt], nxt[2 * kIt];
+        auto load = [&](int64_t uu, int kk, int hh, float4(&v)[2 * kIt]) {
+            const int64_t w0 = (uu / n_mpairs) * TN;
             const int k = kk * kKc + hh * 32 + g * 8;
 #pragma unroll
-            for (int it = 0; it < 4; ++it) {
+            for (int it = 0; it < kIt; ++it) {
                 const int64_t w = w0 + it * 64 + rw;
                 const float* p = pos + (size_t)w * K + k;
                 const bool in = w < nwalk;
@@ -441,10 +476,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             if (h == 0 &&
                 !mbar_wait(bar(kBarBEmpty + sb), (uint32_t)((i / kBStages) & 1) ^ 1u, abort_flag, err, true))
                 break;
-            uint8_t* xh = sm + kOffXb + (uint32_t)sb * 2 * kXbBytes;
-            uint8_t* xl = xh + kXbBytes;
+            uint8_t* xh = sm + kOffXb + (uint32_t)sb * 2 * kXbBytes<TN>;
+            uint8_t* xl = xh + kXbBytes<TN>;
 #pragma unroll
-            for (int it = 0; it < 4; ++it) {
+            for (int it = 0; it < kIt; ++it) {
                 const int n = it * 64 + rw;
                 const float4 a = cur[2 * it], b = cur[2 * it + 1];
                 uint4 hi, lo;
@@ -462,7 +497,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 ++i;
             }
 #pragma unroll
-            for (int e = 0; e < 8; ++e) cur[e] = nxt[e];
+            for (int e = 0; e < 2 * kIt; ++e) cur[e] = nxt[e];
             u = un;
             kc = kn;
             h = hn;
@@ -470,17 +505,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     } else if (warp == kWarpMma) {
         // MMA issue
         if (lane == 0) {
-            int64_t i = 0, j = 0, t = 0;
+            int64_t i = 0, j = 0;
+            uint32_t t0 = 0u, t1 = 0u;   // units each accumulator has taken (PAIRS: alike)
             bool ok = true;
-            for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++t) {
+            for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+                const int na = tiles((int)(u % n_mpairs));
                 for (int kc = 0; kc < nk && ok; ++kc, ++i) {
                     const int sb = (int)(i % kBStages);
                     if (!(ok = mbar_wait(bar(kBarConv + sb), (uint32_t)((i / kBStages) & 1), abort_flag, err, true))) break;
-                    const uint32_t xa = sbase + kOffXb + (uint32_t)sb * 2 * kXbBytes;
-                    for (int a = 0; a < 2; ++a, ++j) {
+                    const uint32_t xa = sbase + kOffXb + (uint32_t)sb * 2 * kXbBytes<TN>;
+                    for (int a = 0; a < na; ++a, ++j) {
                         if (kc == 0) {
-                            // the epilogue has read this tile's accumulator of the previous unit
-                            if (!(ok = mbar_wait(bar(kBarAccEmpty + a), (uint32_t)(t & 1) ^ 1u, abort_flag, err, true)))
+                            // the epilogue has read what this accumulator last held
+                            if (!(ok = mbar_wait(bar(kBarAccEmpty + a), ((a ? t1 : t0) & 1u) ^ 1u, abort_flag, err, true)))
                                 break;
                         }
                         const int sg = (int)(j % kGStages);
@@ -488,21 +525,23 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                             break;
                         tc_fence_after();
                         const uint32_t ga = sbase + kOffG + (uint32_t)sg * 2 * kGBytes;
-                        const uint32_t d = tmem + (uint32_t)a * kTileN;
+                        const uint32_t d = tmem + (uint32_t)a * TN;
 #pragma unroll
                         for (int ks = 0; ks < kKc / 16; ++ks) {
                             const uint32_t dk = (uint32_t)ks * 32;        // K = 16 BF16 = 32 B into the rows
                             const uint64_t a_hi = smem_desc(ga + dk), a_lo = smem_desc(ga + kGBytes + dk);
-                            const uint64_t b_hi = smem_desc(xa + dk), b_lo = smem_desc(xa + kXbBytes + dk);
-                            umma_bf16(d, a_hi, b_hi, (kc > 0 || ks > 0) ? 1u : 0u);
-                            umma_bf16(d, a_hi, b_lo, 1u);
-                            umma_bf16(d, a_lo, b_hi, 1u);
+                            const uint64_t b_hi = smem_desc(xa + dk), b_lo = smem_desc(xa + kXbBytes<TN> + dk);
+                            umma_bf16<TN>(d, a_hi, b_hi, (kc > 0 || ks > 0) ? 1u : 0u);
+                            umma_bf16<TN>(d, a_hi, b_lo, 1u);
+                            umma_bf16<TN>(d, a_lo, b_hi, 1u);
                         }
                         umma_commit(bar(kBarGEmpty + sg));   // this waveform chunk is free when these are done
                         if (kc == nk - 1) umma_commit(bar(kBarAccFull + a));
                     }
                     if (ok) umma_commit(bar(kBarBEmpty + sb));   // the position chunk too
                 }
+                ++t0;
+                t1 += (uint32_t)(PAIRS || na == 2);
             }
             // every MMA issued has completed before the tensor memory is freed
             umma_commit(bar(kBarFin));
@@ -511,19 +550,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     } else {
         // epilogue: warp q reads TMEM lanes 32q .. 32q + 31 (waveform rows)
         const int q = warp - kWarpEpi;   // = warp % 4, the lane quarter this warp may access
-        int64_t t = 0;
+        uint32_t t0 = 0u, t1 = 0u;
         bool ok = true;
-        for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++t) {
-            const int mp = (int)(u % n_mpairs);
-            const int64_t n0 = (u / n_mpairs) * kTileN;
-            for (int a = 0; a < 2; ++a) {
-                if (!(ok = mbar_wait(bar(kBarAccFull + a), (uint32_t)(t & 1), abort_flag, err, true))) break;
+        for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+            const int mp = (int)(u % n_mpairs), na = tiles(mp);
+            const int64_t n0 = (u / n_mpairs) * TN;
+            for (int a = 0; a < na; ++a) {
+                if (!(ok = mbar_wait(bar(kBarAccFull + a), (a ? t1 : t0) & 1u, abort_flag, err, true))) break;
                 __syncwarp();   // tcgen05.ld is warp-wide
                 tc_fence_after();
-                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)a * kTileN;
+                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)a * TN;
                 double CS = 0.0, SN = 0.0;
 #pragma unroll 1
-                for (int c = 0; c < kTileN / 32; ++c) {
+                for (int c = 0; c < TN / 32; ++c) {
                     uint32_t r[32];
                     tmem_ld32(taddr + (uint32_t)c * 32, r);
                     const int64_t nb = n0 + c * 32;
@@ -560,6 +599,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     atomicAdd(out + 2 * jw + 1, SN);
                 }
             }
+            ++t0;
+            t1 += (uint32_t)(PAIRS || na == 2);
         }
     }
 
@@ -567,7 +608,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     __syncthreads();
     tc_fence_after();
     if (warp == kWarpMma)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols<TN>) : "memory");
 }
 
 // Positions already split by the walk (RMS_CONTRACT_BF16X3_PRESPLIT): the same
@@ -575,10 +616,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 constexpr int kPsWarpX = 0, kPsWarpG = 1, kPsWarpMma = 2, kPsWarpEpi = 4;
 constexpr int kPsThreads = 256;
 
+template <int TN, bool PAIRS>
 __global__ void __launch_bounds__(kPsThreads, 1)
     contract_presplit_kernel(const __grid_constant__ CUtensorMap xhi, const __grid_constant__ CUtensorMap xlo,
                              const uint8_t* __restrict__ gpack, int64_t nwalk,
                        int nwave, int nk, int n_mpairs, int64_t nunits, double* __restrict__ out, int* err) {
+    // waveform tiles of a pair: the last pair's second tile may hold no waveform
+    // (PAIRS: never, and no role looks; 1 % of a full contraction)
+    auto tiles = [&](int mp) { return PAIRS || (2 * mp + 1) * kTileM < nwave ? 2 : 1; };
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
@@ -606,7 +651,7 @@ __global__ void __launch_bounds__(kPsThreads, 1)
     }
     if (warp == kPsWarpMma) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(sbase + kOffTmemSlot), "r"(kTmemCols)
+                     ::"r"(sbase + kOffTmemSlot), "r"(kTmemCols<TN>)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -622,9 +667,9 @@ __global__ void __launch_bounds__(kPsThreads, 1)
             int64_t j = 0;
             bool ok = true;
             for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
-                const int mp = (int)(u % n_mpairs);
+                const int mp = (int)(u % n_mpairs), na = tiles(mp);
                 for (int kc = 0; kc < nk && ok; ++kc) {
-                    for (int a = 0; a < 2; ++a, ++j) {
+                    for (int a = 0; a < na; ++a, ++j) {
                         const int s = (int)(j % kGStages);
                         if (!(ok = mbar_wait(bar(kBarGEmpty + s), (uint32_t)((j / kGStages) & 1) ^ 1u, abort_flag, err,
                                              true)))
@@ -647,15 +692,15 @@ __global__ void __launch_bounds__(kPsThreads, 1)
             int64_t i = 0;
             bool ok = true;
             for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
-                const int y = (int)((u / n_mpairs) * kTileN);
+                const int y = (int)((u / n_mpairs) * TN);
                 for (int kc = 0; kc < nk; ++kc, ++i) {
                     const int sb = (int)(i % kBStages);
                     if (!(ok = mbar_wait(bar(kBarBEmpty + sb), (uint32_t)((i / kBStages) & 1) ^ 1u, abort_flag, err, true)))
                         break;
-                    const uint32_t dst = sbase + kOffXb + (uint32_t)sb * 2 * kXbBytes;
-                    mbar_arrive_tx(bar(kBarConv + sb), 2 * kXbBytes);
+                    const uint32_t dst = sbase + kOffXb + (uint32_t)sb * 2 * kXbBytes<TN>;
+                    mbar_arrive_tx(bar(kBarConv + sb), 2 * kXbBytes<TN>);
                     tma_load_2d(dst, &xhi, kc * kKc, y, bar(kBarConv + sb));
-                    tma_load_2d(dst + kXbBytes, &xlo, kc * kKc, y, bar(kBarConv + sb));
+                    tma_load_2d(dst + kXbBytes<TN>, &xlo, kc * kKc, y, bar(kBarConv + sb));
                 }
             }
             for (int64_t jj = i > kBStages ? i - kBStages : 0; jj < i; ++jj)
@@ -664,17 +709,19 @@ __global__ void __launch_bounds__(kPsThreads, 1)
     } else if (warp == kPsWarpMma) {
         // MMA issue
         if (lane == 0) {
-            int64_t i = 0, j = 0, t = 0;
+            int64_t i = 0, j = 0;
+            uint32_t t0 = 0u, t1 = 0u;   // units each accumulator has taken (PAIRS: alike)
             bool ok = true;
-            for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++t) {
+            for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+                const int na = tiles((int)(u % n_mpairs));
                 for (int kc = 0; kc < nk && ok; ++kc, ++i) {
                     const int sb = (int)(i % kBStages);
                     if (!(ok = mbar_wait(bar(kBarConv + sb), (uint32_t)((i / kBStages) & 1), abort_flag, err, true))) break;
-                    const uint32_t xa = sbase + kOffXb + (uint32_t)sb * 2 * kXbBytes;
-                    for (int a = 0; a < 2; ++a, ++j) {
+                    const uint32_t xa = sbase + kOffXb + (uint32_t)sb * 2 * kXbBytes<TN>;
+                    for (int a = 0; a < na; ++a, ++j) {
                         if (kc == 0) {
-                            // the epilogue has read this tile's accumulator of the previous unit
-                            if (!(ok = mbar_wait(bar(kBarAccEmpty + a), (uint32_t)(t & 1) ^ 1u, abort_flag, err, true)))
+                            // the epilogue has read what this accumulator last held
+                            if (!(ok = mbar_wait(bar(kBarAccEmpty + a), ((a ? t1 : t0) & 1u) ^ 1u, abort_flag, err, true)))
                                 break;
                         }
                         const int sg = (int)(j % kGStages);
@@ -682,21 +729,23 @@ __global__ void __launch_bounds__(kPsThreads, 1)
                             break;
                         tc_fence_after();
                         const uint32_t ga = sbase + kOffG + (uint32_t)sg * 2 * kGBytes;
-                        const uint32_t d = tmem + (uint32_t)a * kTileN;
+                        const uint32_t d = tmem + (uint32_t)a * TN;
 #pragma unroll
                         for (int ks = 0; ks < kKc / 16; ++ks) {
                             const uint32_t dk = (uint32_t)ks * 32;        // K = 16 BF16 = 32 B into the rows
                             const uint64_t a_hi = smem_desc(ga + dk), a_lo = smem_desc(ga + kGBytes + dk);
-                            const uint64_t b_hi = smem_desc(xa + dk), b_lo = smem_desc(xa + kXbBytes + dk);
-                            umma_bf16(d, a_hi, b_hi, (kc > 0 || ks > 0) ? 1u : 0u);
-                            umma_bf16(d, a_hi, b_lo, 1u);
-                            umma_bf16(d, a_lo, b_hi, 1u);
+                            const uint64_t b_hi = smem_desc(xa + dk), b_lo = smem_desc(xa + kXbBytes<TN> + dk);
+                            umma_bf16<TN>(d, a_hi, b_hi, (kc > 0 || ks > 0) ? 1u : 0u);
+                            umma_bf16<TN>(d, a_hi, b_lo, 1u);
+                            umma_bf16<TN>(d, a_lo, b_hi, 1u);
                         }
                         umma_commit(bar(kBarGEmpty + sg));   // this waveform chunk is free when these are done
                         if (kc == nk - 1) umma_commit(bar(kBarAccFull + a));
                     }
                     if (ok) umma_commit(bar(kBarBEmpty + sb));   // the position chunk too
                 }
+                ++t0;
+                t1 += (uint32_t)(PAIRS || na == 2);
             }
             // every MMA issued has completed before the tensor memory is freed
             umma_commit(bar(kBarFin));
@@ -705,19 +754,19 @@ __global__ void __launch_bounds__(kPsThreads, 1)
     } else if (warp >= kPsWarpEpi) {
         // epilogue: warp q reads TMEM lanes 32q .. 32q + 31 (waveform rows)
         const int q = warp - kPsWarpEpi;   // = warp % 4, the lane quarter this warp may access
-        int64_t t = 0;
+        uint32_t t0 = 0u, t1 = 0u;
         bool ok = true;
-        for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x, ++t) {
-            const int mp = (int)(u % n_mpairs);
-            const int64_t n0 = (u / n_mpairs) * kTileN;
-            for (int a = 0; a < 2; ++a) {
-                if (!(ok = mbar_wait(bar(kBarAccFull + a), (uint32_t)(t & 1), abort_flag, err, true))) break;
+        for (int64_t u = blockIdx.x; u < nunits && ok; u += gridDim.x) {
+            const int mp = (int)(u % n_mpairs), na = tiles(mp);
+            const int64_t n0 = (u / n_mpairs) * TN;
+            for (int a = 0; a < na; ++a) {
+                if (!(ok = mbar_wait(bar(kBarAccFull + a), (a ? t1 : t0) & 1u, abort_flag, err, true))) break;
                 __syncwarp();   // tcgen05.ld is warp-wide
                 tc_fence_after();
-                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)a * kTileN;
+                const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)a * TN;
                 double CS = 0.0, SN = 0.0;
 #pragma unroll 1
-                for (int c = 0; c < kTileN / 32; ++c) {
+                for (int c = 0; c < TN / 32; ++c) {
                     uint32_t r[32];
                     tmem_ld32(taddr + (uint32_t)c * 32, r);
                     const int64_t nb = n0 + c * 32;
@@ -754,6 +803,8 @@ __global__ void __launch_bounds__(kPsThreads, 1)
                     atomicAdd(out + 2 * jw + 1, SN);
                 }
             }
+            ++t0;
+            t1 += (uint32_t)(PAIRS || na == 2);
         }
     }
 
@@ -761,7 +812,7 @@ __global__ void __launch_bounds__(kPsThreads, 1)
     __syncthreads();
     tc_fence_after();
     if (warp == kPsWarpMma)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols<TN>) : "memory");
 }
 
 // ----------------------------------------------------------------------------
@@ -784,13 +835,92 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// per-device workspace: packed waveforms and the error word
+// A call's workspace: packed waveforms and the error word on the device, and a
+// pinned word to read the latter into.  Calls of several threads or streams each
+// take their own; at most kMostFree wait for the next ones.
 struct Workspace {
     void* p = nullptr;
     size_t bytes = 0;
+    int* herr = nullptr;
+    int device = -1;
 };
 std::mutex g_ws_mu;
-std::vector<Workspace> g_ws;
+std::vector<Workspace> g_ws_free;
+constexpr size_t kMostFree = 4;
+
+void free_workspace(const Workspace& w) {
+    if (w.p) cudaFree(w.p);   // waits for the device
+    if (w.herr) cudaFreeHost(w.herr);
+}
+
+bool take_workspace(size_t bytes, int device, Workspace& w) {
+    {
+        std::lock_guard<std::mutex> lk(g_ws_mu);
+        int pick = -1;   // one that is large enough, else any (it is grown)
+        for (int k = 0; k < (int)g_ws_free.size(); ++k)
+            if (g_ws_free[k].device == device && (pick < 0 || g_ws_free[k].bytes >= bytes)) pick = k;
+        if (pick >= 0) {
+            w = g_ws_free[pick];
+            g_ws_free.erase(g_ws_free.begin() + pick);
+        }
+    }
+    if (w.p && w.bytes >= bytes) return true;
+    free_workspace(w);
+    w = Workspace{};
+    w.device = device;
+    w.bytes = bytes;
+    if (cudaMalloc(&w.p, bytes) == cudaSuccess && cudaMallocHost(reinterpret_cast<void**>(&w.herr), sizeof(int)) == cudaSuccess)
+        return true;
+    free_workspace(w);
+    w = Workspace{};
+    return false;
+}
+
+// Returns a call's workspace; `idle`: the stream has been waited for.
+struct WorkspaceGuard {
+    Workspace w;
+    bool idle = false;
+    ~WorkspaceGuard() {
+        if (!w.p) return;
+        if (idle) {
+            std::lock_guard<std::mutex> lk(g_ws_mu);
+            if (g_ws_free.size() < kMostFree) {
+                try {
+                    g_ws_free.push_back(w);
+                    return;
+                } catch (const std::bad_alloc&) {
+                }
+            }
+        }
+        free_workspace(w);
+    }
+};
+
+// Walkers per tile: the one of 256, 128, 64 whose rounds of units end first.  A
+// narrower MMA reads as much of the waveforms for fewer walkers: a walker costs
+// 1.4 times as much at 128 and 2.1 times at 64 (1e6 walkers x 768 x 1024: 5.1 ms
+// at 256, 10.9 at 64), so they win only where 256 leaves SMs idle (4763 walkers x
+// 480 x 120: 42 us at 256, 20 at 64).
+int walkers_per_tile(int64_t nwalk, int n_mpairs, int sms) {
+    int best = kTileNMax;
+    double least = -1.0;
+    for (int tn = kTileNMax; tn >= 64; tn >>= 1) {
+        const int64_t units = (int64_t)n_mpairs * ((nwalk + tn - 1) / tn);
+        const double t = (double)((units + sms - 1) / sms * tn) * (tn == 256 ? 1.0 : (tn == 128 ? 1.4 : 2.1));
+        if (least < 0 || t < least) {
+            best = tn;
+            least = t;
+        }
+    }
+    return best;
+}
+
+template <class F>
+auto by_tile(int tn, bool pairs, F&& f) {
+    if (tn == 64) return f.template operator()<64, false>();
+    if (tn == 128) return f.template operator()<128, false>();
+    return pairs ? f.template operator()<256, true>() : f.template operator()<256, false>();
+}
 
 }  // namespace
 
@@ -822,10 +952,9 @@ int contract_phases(const float* d_pos, int64_t nwalk, int nbins, const float* d
     } ev;
     if (kernel_ms && (cudaEventCreate(&ev.a) != cudaSuccess || cudaEventCreate(&ev.b) != cudaSuccess))
         return fail(RMS_ERR_CUDA, "events");
-    if (cudaMemsetAsync(d_out, 0, sizeof(double) * 2 * (size_t)nwave, st) != cudaSuccess)
-        return fail(RMS_ERR_CUDA, "clearing the output");
-
     if (method == RMS_CONTRACT_FP32) {
+        if (cudaMemsetAsync(d_out, 0, sizeof(double) * 2 * (size_t)nwave, st) != cudaSuccess)
+            return fail(RMS_ERR_CUDA, "clearing the output");
         const int n_mtiles = (nwave + kF32Tile - 1) / kF32Tile;
         const int64_t blocks = (int64_t)n_mtiles * ((nwalk + kF32Tile - 1) / kF32Tile);
         if (blocks > 0x7fffffff) return fail(RMS_ERR_RANGE, "too many walkers");
@@ -843,36 +972,29 @@ int contract_phases(const float* d_pos, int64_t nwalk, int nbins, const float* d
         const int n_mpairs = (nwave + 2 * kTileM - 1) / (2 * kTileM);
         const int n_mtiles = 2 * n_mpairs;   // the last tiles' rows past nwave are zero
         const size_t gbytes = (size_t)n_mtiles * nk * 2 * kGBytes;
-        void* ws;
-        {
-            std::lock_guard<std::mutex> lk(g_ws_mu);
-            if ((int)g_ws.size() <= dev) g_ws.resize(dev + 1);
-            Workspace& w = g_ws[dev];
-            if (w.bytes < gbytes + 256) {
-                if (w.p) cudaFree(w.p);
-                w.p = nullptr;
-                w.bytes = 0;
-                if (cudaMalloc(&w.p, gbytes + 256) != cudaSuccess) return fail(RMS_ERR_NOMEM, "workspace");
-                w.bytes = gbytes + 256;
-            }
-            ws = w.p;
-        }
-        uint8_t* gpack = static_cast<uint8_t*>(ws);
+        WorkspaceGuard ws;
+        if (!take_workspace(gbytes + 256, dev, ws.w)) return fail(RMS_ERR_NOMEM, "workspace");
+        uint8_t* gpack = static_cast<uint8_t*>(ws.w.p);
         int* d_err = reinterpret_cast<int*>(gpack + gbytes);
-        if (cudaMemsetAsync(d_err, 0, sizeof(int), st) != cudaSuccess) return fail(RMS_ERR_CUDA, "error word");
-        pack_waves_kernel<<<1024, 256, 0, st>>>(d_wave, nwave, K, nk, n_mtiles, gpack);
+        const int64_t items = (int64_t)n_mtiles * kTileM * nk * (kKc / 8);
+        pack_waves_kernel<<<(unsigned)std::min<int64_t>(1024, (items + 255) / 256), 256, 0, st>>>(
+            d_wave, nwave, K, nk, n_mtiles, gpack, d_err, d_out);
         if (cudaGetLastError() != cudaSuccess) return fail(RMS_ERR_CUDA, "waveform packing launch");
 
         static std::once_flag attr_once;
         static cudaError_t attr_err = cudaSuccess;
         std::call_once(attr_once, [] {
-            attr_err = cudaFuncSetAttribute(contract_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)kSmemBytes);
-            if (attr_err == cudaSuccess)
-                attr_err = cudaFuncSetAttribute(contract_presplit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)kSmemBytes);
+            for (int tn : {64, 128, 256, 257})   // (257: 256 with full pairs)
+                by_tile(tn, tn == 257, [&]<int TN, bool PAIRS>() {
+                    for (const void* k : {(const void*)contract_tc_kernel<TN, PAIRS>,
+                                          (const void*)contract_presplit_kernel<TN, PAIRS>})
+                        if (attr_err == cudaSuccess)
+                            attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                            (int)kSmemBytes);
+                });
         });
         if (attr_err != cudaSuccess) return fail(RMS_ERR_CUDA, "shared memory attribute");
+        const int tn = walkers_per_tile(nwalk, n_mpairs, sms);
         CUtensorMap mhi, mlo;
         if (presplit) {
             EncodeTiledFn enc = encode_fn();
@@ -880,7 +1002,7 @@ int contract_phases(const float* d_pos, int64_t nwalk, int nbins, const float* d
             if (nwalk > 0x7fffffffll) return fail(RMS_ERR_RANGE, "too many walkers for one tensor map");
             const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)nwalk};
             const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-            const cuuint32_t box[2] = {(cuuint32_t)kKc, (cuuint32_t)kTileN};
+            const cuuint32_t box[2] = {(cuuint32_t)kKc, (cuuint32_t)tn};
             const cuuint32_t estr[2] = {1, 1};
             uint8_t* hi = reinterpret_cast<uint8_t*>(const_cast<float*>(d_pos));
             uint8_t* lo = hi + (size_t)nwalk * K * 2;
@@ -890,22 +1012,24 @@ int contract_phases(const float* d_pos, int64_t nwalk, int nbins, const float* d
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                     return fail(RMS_ERR_CUDA, "tensor map of the positions");
         }
-        const int64_t nunits = (int64_t)n_mpairs * ((nwalk + kTileN - 1) / kTileN);
+        const int64_t nunits = (int64_t)n_mpairs * ((nwalk + tn - 1) / tn);
         const int grid = (int)std::min<int64_t>(nunits, sms);
         if (ev.a) cudaEventRecord(ev.a, st);
-        if (presplit)
-            contract_presplit_kernel<<<grid, kPsThreads, kSmemBytes, st>>>(mhi, mlo, gpack, nwalk, nwave, nk, n_mpairs,
-                                                                           nunits, d_out, d_err);
-        else
-            contract_tc_kernel<<<grid, kTcThreads, kSmemBytes, st>>>(d_pos, K, gpack, nwalk, nwave, nk, n_mpairs,
-                                                                     nunits, d_out, d_err);
+        by_tile(tn, (nwave + kTileM - 1) / kTileM % 2 == 0, [&]<int TN, bool PAIRS>() {
+            if (presplit)
+                contract_presplit_kernel<TN, PAIRS><<<grid, kPsThreads, kSmemBytes, st>>>(mhi, mlo, gpack, nwalk, nwave, nk,
+                                                                                   n_mpairs, nunits, d_out, d_err);
+            else
+                contract_tc_kernel<TN, PAIRS><<<grid, kTcThreads, kSmemBytes, st>>>(d_pos, K, gpack, nwalk, nwave, nk, n_mpairs,
+                                                                             nunits, d_out, d_err);
+        });
         if (ev.b) cudaEventRecord(ev.b, st);
         if (cudaGetLastError() != cudaSuccess) return fail(RMS_ERR_CUDA, "tensor-core contraction launch");
-        int herr = 0;
-        if (cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        if (cudaMemcpyAsync(ws.w.herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return fail(RMS_ERR_CUDA, "tensor-core contraction");
-        if (herr & kErrTimeout) return fail(RMS_ERR_TIMEOUT, "a pipeline wait of the tensor-core contraction ran out");
+        ws.idle = true;
+        if (*ws.w.herr & kErrTimeout) return fail(RMS_ERR_TIMEOUT, "a pipeline wait of the tensor-core contraction ran out");
     }
     if (kernel_ms && (cudaEventElapsedTime(kernel_ms, ev.a, ev.b) != cudaSuccess))
         return fail(RMS_ERR_CUDA, "contraction timing");
