@@ -358,6 +358,8 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
             float B0 = 0.0f, B1 = 0.0f, B2 = 0.0f;  // bin sums of the tangent
             int bin = i_start / a.bin_steps, next_bin = (i_start / a.bin_steps + 1) * a.bin_steps;
             fetch_bin(tab_b, a, bin, lane, pass < 2);
+            // the step that ends the FP32 sums: every 32nd, and every bin's last
+            int next_fold = min((i_start & ~31) + 32, next_bin);
             float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f, q3 = 0.0f;   // the split walk's direction stream
             int phase = 0;
             uint32_t dblk = (uint32_t)(i_start / 3);
@@ -397,11 +399,10 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                     float u[6];
                     dir_fields(dir_block(dblk++, key0, key1, wlo, whi), u);
                     u1 = u[0]; u2 = u[1]; q0 = u[2]; q1 = u[3]; q2 = u[4]; q3 = u[5];
-                    phase = 1;
-                } else if (phase == 1) {
-                    u1 = q0; u2 = q1; phase = 2;
+                    phase = 2;
                 } else {
-                    u1 = q2; u2 = q3; phase = 0;
+                    u1 = q0; u2 = q1; q0 = q2; q1 = q3;
+                    --phase;
                 }
                 if (active) {
                     float v0, v1, v2;
@@ -416,8 +417,10 @@ __global__ void __launch_bounds__(kAdjBlock, adj_min_blocks(JAC, FORM)) adjoint_
                 p1 += D1 + (o1 - Fm1);
                 p2 += D2 + (o2 - Fm2);
                 if (p1st) { B0 += h.T0; B1 += h.T1; B2 += h.T2; }
-                const bool event = (i + 1 == next_bin);
-                if (event || (i & 31) == 31) {
+                bool event = false;
+                if (i + 1 == next_fold) {
+                    event = (i + 1 == next_bin);
+                    next_fold = min(((i + 1) & ~31) + 32, event ? next_bin + a.bin_steps : next_bin);
                     P0 += (double)p0; P1 += (double)p1; P2 += (double)p2;
                     p0 = p1 = p2 = 0.0f;
                     w64 += (double)wk.w32;

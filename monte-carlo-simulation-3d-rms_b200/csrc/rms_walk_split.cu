@@ -496,10 +496,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
         int rec = 0, left = 1;
         int evi = 0;   // next PGSE event, or current waveform bin
         int next_ev = pgse ? (a.nevents > 0 ? a.ev_step[0] : -1) : (wave ? a.bin_steps : -1);
+        // the step that ends the FP32 sums: every 32nd, and every event
+        int next_fold = next_ev > 0 ? min(32, next_ev) : 32;
         if (sums)
             for (int k = 0; k < (pgse ? a.npairs * 3 : a.nwave); ++k) a.vscr[(size_t)k * nthr + gtid] = 0.0;
         // direction uniforms: one Philox block per three steps, in lock step;
-        // the next two steps' pairs wait in q0..q3
+        // the next two steps' pairs wait in q0..q3 and move up (phase: how many)
         float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f, q3 = 0.0f;
         int phase = 0;
         uint32_t dblk = 0u;
@@ -511,11 +513,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                 float u[6];
                 dir_fields(dir_block(dblk++, key0, key1, wlo, whi), u);
                 u1 = u[0]; u2 = u[1]; q0 = u[2]; q1 = u[3]; q2 = u[4]; q3 = u[5];
-                phase = 1;
-            } else if (phase == 1) {
-                u1 = q0; u2 = q1; phase = 2;
+                phase = 2;
             } else {
-                u1 = q2; u2 = q3; phase = 0;
+                u1 = q0; u2 = q1; q0 = q2; q1 = q3;
+                --phase;
             }
             if (active) {
                 // RULE != 0: the step's start, restored when a membrane turns the step back
@@ -550,10 +551,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                 p0 += D0 + (o0 - Fm0);
                 p1 += D1 + (o1 - Fm1);
                 p2 += D2 + (o2 - Fm2);
-                const bool event = (i + 1 == next_ev);
-                if (event || (i & 31) == 31) {
+                bool event = false;
+                if (i + 1 == next_fold) {
                     P0 += (double)p0; P1 += (double)p1; P2 += (double)p2;
                     p0 = p1 = p2 = 0.0f;
+                    event = (i + 1 == next_ev);
+                    next_fold = ((i + 1) & ~31) + 32;
+                    if (!event && next_ev > 0) next_fold = min(next_fold, next_ev);
                 }
                 if (event && wave) {
                     wave_bin(a.wave, a.nwave, evi, P0, P1, P2, (double)AXF(res), a.vscr + gtid, nthr, a.traj,
@@ -562,6 +566,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                     P0 = P1 = P2 = 0.0;
                     ++evi;
                     next_ev += a.bin_steps;
+                    next_fold = min(next_fold, next_ev);
                 } else if (event) {
                     do {
                         const double cf = a.ev_coef[evi];
@@ -572,6 +577,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) walk_split_kernel(const WalkArgs 
                         ++evi;
                     } while (evi < a.nevents && a.ev_step[evi] == i + 1);
                     next_ev = (evi < a.nevents) ? a.ev_step[evi] : -1;
+                    if (next_ev > 0) next_fold = min(next_fold, next_ev);
                 }
             }
 
