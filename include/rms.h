@@ -63,8 +63,8 @@ extern "C" {
  *  SPLIT:  int32 voxel index + FP32 in-voxel offset, FP32 uniforms, FP64
  *          cross-walker sums; statistically equal to COMPAT.
  *  Repeatability: COMPAT sums each record's per-warp rows in a fixed order,
- *  so a rerun with the same seed is identical bit for bit; SPLIT adds the
- *  warps' rows into the totals with FP64 atomics, so a rerun has the same
+ *  so a rerun with the same seed is identical bit for bit; SPLIT adds its
+ *  records into the totals with FP64 atomics, so a rerun has the same
  *  walkers and compartment counts and equal sums up to their order (about
  *  1e-15 relative). */
 #define RMS_PREC_COMPAT 0

@@ -118,8 +118,9 @@ bool split_variant_walks(int variant, int mode, int rule);   // variants past th
 int split_variant_block(int variant);   // threads per block of a launch variant
 int split_variant_minb(int variant);    // its minimum resident blocks per SM
 // The split walk's lattice: (n1+2) x (n2+2) x (n3+2) with a wall-code border;
-// 4 bits per voxel (3-bit label + free-flight flag) when Nc <= 7 (every split
-// walk, the no-allocation one included), else one byte.
+// one byte per voxel (7-bit label + free-flight flag), or 4 bits (3-bit label +
+// flag, Nc <= 7): the no-allocation walk's, and other launches' by lattice size
+// (launch_cell_bits in rms_api.cpp).  split_lattice_bits: the narrowest for Nc.
 int split_lattice_bits(int nc);
 size_t padded_lattice_bytes(int n1, int n2, int n3, int bits);
 // mirror: flag voxels at the lattice's faces too (mirror walls; see pad_pack_kernel)

@@ -17,7 +17,7 @@
 // (rms_walk_split.cu, rms_reduce.cu), launched on that scratch.  The grid is
 // sized so the per-warp rows fit in the scratch; a job whose fixed tables or
 // single block of rows do not fit is refused with RMS_ERR_RANGE.  The walk
-// reads the same padded, packed lattice as rms_sim_run (4 bits per voxel with
+// reads the padded, packed lattice rms_sim_run takes for large ones (4 bits per voxel with
 // the free-flight flags, Nc <= 7), built in the scratch too: 68 MB for
 // 256x256x2048.  Same lattice, same kernel, same walkers: the results equal
 // rms_sim_run's up to the order of the final sums.  The caller's lattice is

@@ -22,9 +22,9 @@
 //    one straight line -- a floor per axis instead of the face loop.  It is
 //    the face loop's own outcome (every face on the way is a same-label face,
 //    always crossed) with at most three crossings, within the nite = 4 cap;
-//  - labels packed 4 bits per voxel (3-bit label, wall = 7, plus the flag;
-//    a padded 256x256x2048 lattice is 68 MB and stays in the 126 MB L2), or
-//    one byte for Nc = 8;
+//  - labels one byte per voxel (7-bit label, wall = 127, plus the flag), or
+//    packed 4 bits (3-bit label, wall = 7, plus the flag) where that keeps a
+//    large lattice in the 126 MB L2 (a padded 256x256x2048 one is 68 MB);
 //  - FP32 uniforms (21-bit), one Philox4x32-10 block per three steps;
 //    hardware sine/cosine and reciprocal for the direction and face times;
 //  - per-walker sums that grow over the walk (T2 exponent, PGSE displacement
@@ -195,7 +195,7 @@ __device__ __noinline__ void wave_final(const double* ph, int nthr, int nwave, d
 // warp-record costs five loads, 24 conversions and adds and ~30 paired products
 // (__fmul2_rn: two walkers an instruction), no shuffle.  1e6 walkers x 2000
 // steps on a 128x128x900 axon, walk kernel: 12.5 / 35.6 ms with 100 / 2000
-// records before, 12.3 / 27.1 ms now.  KR = 8 up to 256 threads a block (4.2 KB
+// records before, 10.4 / 25.3 ms now (12.3 / 27.1 with the step of that day).  KR = 8 up to 256 threads a block (4.2 KB
 // of staging per warp), 4 above, so the static shared memory stays under 48 KB.
 __host__ __device__ constexpr int rec_batch(int block) { return block <= 256 ? 8 : 4; }
 constexpr int kStageRow = 4 * 32 + 4;   // floats of a staged record: x, y, z, s0 of 32 walkers, and 4 of padding
