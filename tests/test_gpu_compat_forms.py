@@ -95,3 +95,27 @@ def test_b_values_shared_between_lanes(npar, precision):
     for n in (1, 2, 3, 8, 9, 16, 17, 33, 48):
         got = engine.Sim(lab, bval=b[:n], bvec=v[:n], **kw).run(seed=6, precision=precision).outputs()["sigre"]
         assert np.abs(got - full[:, :n]).max() <= 1e-12 * npar, n
+
+
+@pytest.mark.parametrize("D0", [0.0, 5.0, 6.7, 20.0])
+def test_table_that_lets_walkers_into_compartment_0(D0):
+    """Only a permeation table opens compartment 0, whose step length is not held
+    below a voxel (D0 = 20: 1.55 voxels): the same walk, or the same refusal of a
+    segment that finds no face."""
+    lab = lattice()
+    dd, tn, npar = [D0, 2.0, 1.0], 12, 400
+    pij = np.array([[1.0, 0.4, 0.4], [0.5, 1.0, 0.7], [0.5, 0.7, 1.0]])
+    sim = engine.Sim(lab, dt=2e-4, tn=tn, npar=npar, res=0.1, diffusivity=dd, t2=T2, timepoints=tn,
+                     permeation="table", pij=pij, bval=[], bvec=np.zeros((0, 3)))
+    step, t2s, _, td = pyoracle.reference_tables(2e-4, 0.1, dd, T2, tn, tn)
+    job = pyoracle.Job(lab, dt=2e-4, tn=tn, npar=npar, res=0.1, step=step, t2_steps=t2s, pij=pij.ravel(), seed=6,
+                       timepoints=tn, td=td)
+    try:
+        got = sim.run(seed=6, precision="compat", trace_walkers=npar)
+    except engine.RmsError as e:
+        assert D0 == 20.0 and e.code == -4
+        return
+    want = pyoracle.run_oracle(job, trace_walkers=npar)
+    tr = got.trace(npar)
+    assert np.array_equal(tr["voxel"], want["trace"]["voxel"])
+    assert np.array_equal(tr["events"], want["trace"]["events"])
