@@ -171,6 +171,9 @@ __device__ __noinline__ void add_pgse(const WalkArgs& a, int nthr, int t0, doubl
         s = share_sum(s, l);
         if (base + l.item < a.ngrad && l.share == 0) put(sig + j, s, first);
     }
+    // the next tile's walkers clear these sums: every lane has read them by then
+    // (a shuffle orders no memory)
+    __syncwarp();
 }
 
 // What bounds it: FP64 issue (64 lanes per clock and SM) and, below a few warps

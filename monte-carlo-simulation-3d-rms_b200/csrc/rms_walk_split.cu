@@ -369,6 +369,9 @@ __device__ __forceinline__ void add_pgse(const WalkArgs& a, int nthr, int t0, do
         s = share_sum(s, l);
         if (base + l.item < a.ngrad && l.share == 0) add_out<ONE>(sig + j, s);
     }
+    // the next tile's walkers clear these sums: every lane has read them by then
+    // (a shuffle orders no memory)
+    __syncwarp();
 }
 
 // ONE: the no-allocation walk's form -- one axon, whose scalars are read from
