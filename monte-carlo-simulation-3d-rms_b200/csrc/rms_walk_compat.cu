@@ -200,7 +200,9 @@ __global__ void __launch_bounds__(kBlock, MINB) walk_compat_kernel(const __grid_
             s_step[i] = (i < a.nc) ? a.step[i] : 0.0;
             s_t2[i] = (i < a.nc) ? a.t2[i] : 1.0;
             s_rstep[i] = __drcp_rn(s_step[i]);
-            s_rt2[i] = __drcp_rn(s_t2[i]);
+            // (0: weight() divides -- an infinite T2, or one so short or long that 1 / T2
+            // or a quotient leaves the range in which div_by is the division)
+            s_rt2[i] = s_t2[i] > 0x1p-900 && s_t2[i] < 0x1p+900 ? __drcp_rn(s_t2[i]) : 0.0;
         }
     }
     __syncthreads();
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(kBlock, MINB) walk_compat_kernel(const __grid_
             for (int c = 0; c < NCMAX; ++c)
                 if (c < a.nc) {
                     const double tc = s_tc[c][threadIdx.x], y = s_rt2[c];
-                    s = s + (y > 0.0 ? div_by(tc, s_t2[c], y) : tc / s_t2[c]);   // (T2 may be infinite)
+                    s = s + (y > 0.0 ? div_by(tc, s_t2[c], y) : tc / s_t2[c]);
                 }
             return active ? exp(-1.0 * s) : 0.0;
         };
