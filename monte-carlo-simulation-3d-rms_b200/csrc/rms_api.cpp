@@ -44,8 +44,11 @@ constexpr uint64_t kBatchSeedStep = 0x9E3779B97F4A7C15ull;   // seed of batch me
 //    row have passed over is freed, and all of them when an allocation fails;
 //  - blocks go to a request they are at most a quarter (and 1 MB) larger than,
 //    on their own device;
-//  - one mutex; a block enters only after the device has finished everything
-//    (what cudaFree would have waited for), so the next owner may use any stream.
+//  - one mutex; a block enters only when no work on it is in flight (every call
+//    waits for its stream before it returns, on its error paths too: StreamWait),
+//    so the next owner may use any stream.  Nothing here waits for the device:
+//    that would wait for other threads' simulations, and would break a capture
+//    that another thread has begun.
 class BlockCache {
   public:
     explicit BlockCache(bool host) : host_(host), most_(host ? (size_t)256 << 20 : (size_t)4 << 30) {}
@@ -73,14 +76,17 @@ class BlockCache {
             drop([](const Block&) { return true; });
             e = host_ ? cudaMallocHost(p, bytes) : cudaMalloc(p, bytes);
         }
-        if (e != cudaSuccess) *p = nullptr;
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();   // (the next launch's check must not find it)
+            *p = nullptr;
+        }
         *got = bytes;
         return e;
     }
 
-    // the caller's device is the block's
+    // no work on the block is in flight
     void give(void* p, size_t n, int device) {
-        if (cudaDeviceSynchronize() != cudaSuccess || n > most_) {
+        if (n > most_) {
             free_block(p);
             return;
         }
@@ -107,7 +113,9 @@ class BlockCache {
         int device;
         long since;
     };
-    void free_block(void* p) { (void)(host_ ? cudaFreeHost(p) : cudaFree(p)); }
+    void free_block(void* p) {
+        if ((host_ ? cudaFreeHost(p) : cudaFree(p)) != cudaSuccess) (void)cudaGetLastError();
+    }
     template <class F>
     void drop(F which) {
         for (size_t k = 0; k < free_.size();) {
@@ -161,6 +169,24 @@ struct Buffer {
 };
 using DevBuf = Buffer<false>;
 using HostPinned = Buffer<true>;
+
+// Waits for a call's stream when the call returns: a simulation's memory may go
+// to another owner as soon as the call is over, however it ended.  done(): the
+// call has waited itself.
+class StreamWait {
+  public:
+    explicit StreamWait(cudaStream_t st) : st_(st) {}
+    StreamWait(const StreamWait&) = delete;
+    StreamWait& operator=(const StreamWait&) = delete;
+    void done() { waited_ = true; }
+    ~StreamWait() {
+        if (!waited_ && cudaStreamSynchronize(st_) != cudaSuccess) (void)cudaGetLastError();
+    }
+
+  private:
+    cudaStream_t st_;
+    bool waited_ = false;
+};
 }  // namespace
 
 struct rms_device_state {
@@ -515,8 +541,10 @@ int sync_host_labels(rms_sim* s) {
     const size_t n = (size_t)s->n1 * s->n2 * s->n3;
     s->labels.resize(n);
     RMS_CUDA(cudaSetDevice(d->device));
+    StreamWait wait(d->own);
     RMS_CUDA(cudaMemcpyAsync(s->labels.data(), d->labels.p, n, cudaMemcpyDeviceToHost, d->own));
     RMS_CUDA(cudaStreamSynchronize(d->own));
+    wait.done();
     s->host_stale = false;
     return RMS_OK;
 }
@@ -666,6 +694,7 @@ struct LaunchPlan {
     bool multi = false, has_sig = false, wavemode = false;
     int64_t trace_n = 0;
     std::vector<AxonDesc> axons;
+    std::unique_ptr<StreamWait> wait;   // from the first work on st to the end of the call
 };
 
 // Run one launch: COMPAT (one simulation) or SPLIT (one or more simulations,
@@ -693,6 +722,7 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
     rms_device_state* d = s->dev;
     RMS_CUDA(cudaSetDevice(device));
     cudaStream_t st = (o && o->stream) ? (cudaStream_t)o->stream : d->own;
+    p.wait = std::make_unique<StreamWait>(st);
     const int naxons = (int)jobs.size();
 
     int64_t trace_n = (o && o->trace_walkers > 0) ? o->trace_walkers : 0;
@@ -926,6 +956,7 @@ int enqueue_launch(LaunchPlan& p, rms_sim* s, bool events) {
 int finish_launch(std::vector<LaunchJob>& jobs, LaunchPlan& p, bool events) {
     rms_device_state* d = p.d;
     RMS_CUDA(cudaStreamSynchronize(p.st));
+    if (p.wait) p.wait->done();
     const double* h = static_cast<const double*>(d->h_out.p);
     const int herr = *reinterpret_cast<const int*>(h + p.nrow + p.nsig);
     if (herr & kErrInitCap)
@@ -1081,6 +1112,8 @@ int graph_create(rms_sim* const* sims, int n, const rms_run_opts* o, rms_graph**
     LaunchPlan& p = g->plan;
     if (!o->stream) p.st = p.d->own;   // capture needs a stream other than the legacy default stream
     std::memcpy(p.d->h_axons.p, p.axons.data(), sizeof(AxonDesc) * p.naxons);
+    RMS_CUDA(cudaStreamSynchronize(p.st));   // the uploads
+    p.wait.reset();
     RMS_CUDA(cudaStreamBeginCapture(p.st, cudaStreamCaptureModeThreadLocal));
     rc = enqueue_launch(p, g->jobs[0].s, false);
     cudaGraph_t graph = nullptr;
@@ -1107,6 +1140,11 @@ int graph_run(rms_graph* g, uint64_t seed) {
     RMS_CUDA(cudaSetDevice(g->device));
     for (int k = 0; k < p.naxons; ++k) p.axons[k].seed = seed + (uint64_t)k * kBatchSeedStep;
     std::memcpy(p.d->h_axons.p, p.axons.data(), sizeof(AxonDesc) * p.naxons);
+    p.wait = std::make_unique<StreamWait>(p.st);
+    struct Over {
+        LaunchPlan& p;
+        ~Over() { p.wait.reset(); }
+    } over{p};
     RMS_CUDA(cudaEventRecord(p.d->e0, p.st));
     RMS_CUDA(cudaGraphLaunch(g->exec, p.st));
     RMS_CUDA(cudaEventRecord(p.d->e1, p.st));
@@ -1232,6 +1270,7 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
     rms_device_state* d = s->dev;
     RMS_CUDA(cudaSetDevice(device));
     cudaStream_t st = (o && o->stream) ? (cudaStream_t)o->stream : d->own;
+    StreamWait wait(st);
     const int bits = launch_cell_bits({LaunchJob{s, w0, w1, 0}}, s->nc);
     rc = prepare_lattice(s, st, true, bits);
     if (rc) return rc;
@@ -1421,6 +1460,7 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
     RMS_CUDA(cudaMemcpyAsync(dw.data(), d->adj_dwave.p, sizeof(float) * ndw, cudaMemcpyDeviceToHost, st));
     RMS_CUDA(cudaMemcpyAsync(&herr, d->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     RMS_CUDA(cudaStreamSynchronize(st));
+    wait.done();
     if (herr & kErrInitCap)
         return set_error(RMS_ERR_RANGE, "a walker found no labelled voxel within the rejection-sampling cap");
     float ms = 0.f;
@@ -1524,6 +1564,7 @@ int set_lattice_on_device(rms_sim* s, const uint8_t* labels, size_t n) {
     int sms = 0;
     RMS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device));
     unsigned long long hcount[2] = {0, 0};
+    StreamWait wait(d->own);
     RMS_CUDA(cudaMemsetAsync(d->counts.p, 0, sizeof(hcount), d->own));
     RMS_CUDA(cudaMemcpyAsync(d->stage.p, labels, n, cudaMemcpyHostToDevice, d->own));
     // from here the stream reads the caller's buffer: every return waits for it
@@ -1532,6 +1573,7 @@ int set_lattice_on_device(rms_sim* s, const uint8_t* labels, size_t n) {
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(hcount, d->counts.p, sizeof(hcount), cudaMemcpyDeviceToHost, d->own);
     const cudaError_t es = cudaStreamSynchronize(d->own);
+    wait.done();
     if (e != cudaSuccess) return cuda_fail(e, "lattice check");
     if (es != cudaSuccess) return cuda_fail(es, "lattice upload");
     if (hcount[0] || hcount[1] == 0 || (double)hcount[1] / (double)n < 1e-7) {
@@ -1705,6 +1747,7 @@ int rms_sim_set_tube_lattice(rms_sim* s, const double* r2, const double* cx, con
         rms_device_state* d = s->dev;
         RMS_CUDA(cudaSetDevice(device));
         cudaStream_t st = d->own;
+        StreamWait wait(st);
         const size_t nvox = (size_t)s->n1 * s->n2 * s->n3;
         std::vector<double> tab;
         tab.insert(tab.end(), r2, r2 + s->n3);
@@ -1719,6 +1762,7 @@ int rms_sim_set_tube_lattice(rms_sim* s, const double* r2, const double* cx, con
         s->labels.resize(nvox);
         RMS_CUDA(cudaMemcpyAsync(s->labels.data(), d->labels.p, nvox, cudaMemcpyDeviceToHost, st));
         RMS_CUDA(cudaStreamSynchronize(st));
+        wait.done();
         size_t nonzero = 0;
         for (size_t i = 0; i < nvox; ++i) nonzero += s->labels[i] != 0;
         if (nonzero == 0) return set_error(RMS_ERR_RANGE, "the lattice has no labelled voxel");
