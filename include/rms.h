@@ -245,6 +245,14 @@ const char* rms_last_error(void);
 
 void rms_sim_destroy(rms_sim* sim);
 
+/* Device and pinned memory of destroyed simulations and finished contractions is
+ * kept for the next ones (at most 4 GiB and 256 MiB; a block is freed once 256
+ * requests have passed it over, and every block when an allocation of this
+ * library fails).  This gives all of it back, for a program that wants the memory
+ * for something else.  The bytes given back go to *device_bytes and *host_bytes
+ * (each may be NULL). */
+int rms_memory_trim(size_t* device_bytes, size_t* host_bytes);
+
 /* The engine's random stream on the host: n uniforms of walker `walker`
  * (Philox4x32-10; doubles take two words, floats one).  Replaces the draws of
  * curand_uniform_double (main.cu:118-120, 140, 144, 282); a test hook. */

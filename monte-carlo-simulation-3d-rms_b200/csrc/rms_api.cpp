@@ -20,6 +20,7 @@
 #include <thread>
 #include <tuple>
 
+#include "block_cache.h"
 #include "philox.cuh"
 #include "rms_internal.h"
 #include "rms_sim.h"
@@ -36,113 +37,6 @@ constexpr int kSplitVariantDefault = 3;
 constexpr int kMaxGrad = 1 << 16;
 constexpr uint64_t kBatchSeedStep = 0x9E3779B97F4A7C15ull;   // seed of batch member k: seed + k * this
 
-// Memory of closed simulations, kept for the next ones.  A program that makes a
-// simulation per call (a fit through torch makes two per iteration) spent 10 to
-// 40 ms of each in cudaMalloc, cudaMallocHost and their frees: a pass of
-// waveform gradients over 1e5 walkers took 48 to 70 ms, 34.5 with the cache.
-//  - bounded: at most kMost bytes of each kind, a block that 256 requests in a
-//    row have passed over is freed, and all of them when an allocation fails;
-//  - blocks go to a request they are at most a quarter (and 1 MB) larger than,
-//    on their own device;
-//  - one mutex; a block enters only when no work on it is in flight (every call
-//    waits for its stream before it returns, on its error paths too: StreamWait),
-//    so the next owner may use any stream.  Nothing here waits for the device:
-//    that would wait for other threads' simulations, and would break a capture
-//    that another thread has begun.
-class BlockCache {
-  public:
-    explicit BlockCache(bool host) : host_(host), most_(host ? (size_t)256 << 20 : (size_t)4 << 30) {}
-
-    cudaError_t take(size_t bytes, int device, void** p, size_t* got) {
-        std::lock_guard<std::mutex> lk(mu_);
-        ++now_;
-        int best = -1;
-        for (int k = 0; k < (int)free_.size(); ++k) {
-            const Block& b = free_[k];
-            if (b.device == device && b.n >= bytes && b.n <= bytes + bytes / 4 + ((size_t)1 << 20) &&
-                (best < 0 || b.n < free_[best].n))
-                best = k;
-        }
-        if (best >= 0) {
-            *p = free_[best].p;
-            *got = free_[best].n;
-            held_ -= free_[best].n;
-            free_.erase(free_.begin() + best);
-            return cudaSuccess;
-        }
-        cudaError_t e = host_ ? cudaMallocHost(p, bytes) : cudaMalloc(p, bytes);
-        if (e != cudaSuccess && !free_.empty()) {
-            (void)cudaGetLastError();   // a failed allocation is not sticky; clear it
-            drop([](const Block&) { return true; });
-            e = host_ ? cudaMallocHost(p, bytes) : cudaMalloc(p, bytes);
-        }
-        if (e != cudaSuccess) {
-            (void)cudaGetLastError();   // (the next launch's check must not find it)
-            *p = nullptr;
-        }
-        *got = bytes;
-        return e;
-    }
-
-    // no work on the block is in flight
-    void give(void* p, size_t n, int device) {
-        if (n > most_) {
-            free_block(p);
-            return;
-        }
-        std::lock_guard<std::mutex> lk(mu_);
-        try {
-            free_.push_back(Block{p, n, device, now_});
-        } catch (const std::bad_alloc&) {   // (called from destructors and C entries)
-            free_block(p);
-            return;
-        }
-        held_ += n;
-        drop([&](const Block& b) { return now_ - b.since > 256; });
-        while (held_ > most_) {   // the oldest first
-            const long oldest = free_.front().since;
-            bool one = false;
-            drop([&](const Block& b) { return !one && b.since == oldest && (one = true); });
-        }
-    }
-
-  private:
-    struct Block {
-        void* p;
-        size_t n;
-        int device;
-        long since;
-    };
-    void free_block(void* p) {
-        if ((host_ ? cudaFreeHost(p) : cudaFree(p)) != cudaSuccess) (void)cudaGetLastError();
-    }
-    template <class F>
-    void drop(F which) {
-        for (size_t k = 0; k < free_.size();) {
-            if (which(free_[k])) {
-                free_block(free_[k].p);
-                held_ -= free_[k].n;
-                free_.erase(free_.begin() + k);
-            } else {
-                ++k;
-            }
-        }
-    }
-    const bool host_;
-    const size_t most_;
-    std::mutex mu_;
-    std::vector<Block> free_;   // oldest first
-    size_t held_ = 0;
-    long now_ = 0;
-};
-
-// (never destroyed: the CUDA context may be gone before static destructors run)
-BlockCache& block_cache(bool host) {
-    static BlockCache* dev = new BlockCache(false);
-    static BlockCache* pinned = new BlockCache(true);
-    return host ? *pinned : *dev;
-}
-
 // One allocation that only grows, on the device or (HOST) pinned.
 template <bool HOST>
 struct Buffer {
@@ -153,7 +47,7 @@ struct Buffer {
         if (bytes <= n) return cudaSuccess;
         release();
         cudaError_t e = cudaGetDevice(&device);
-        if (e == cudaSuccess) e = block_cache(HOST).take(bytes, device, &p, &n);
+        if (e == cudaSuccess) e = (cudaError_t)rms::block_cache(HOST).take(bytes, device, &p, &n);
         if (e != cudaSuccess) {
             p = nullptr;
             n = 0;
@@ -161,7 +55,7 @@ struct Buffer {
         return e;
     }
     void release() {
-        if (p) block_cache(HOST).give(p, n, device);
+        if (p) rms::block_cache(HOST).give(p, n, device);
         p = nullptr;
         n = 0;
     }
@@ -221,6 +115,27 @@ struct rms_device_state {
 };
 
 namespace rms {
+
+namespace {
+// (an error is returned, not left for the next launch's check to find)
+template <bool HOST>
+int alloc_block(void** p, size_t n) {
+    const cudaError_t e = HOST ? cudaMallocHost(p, n) : cudaMalloc(p, n);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return (int)e;
+}
+template <bool HOST>
+void free_block(void* p) {
+    if ((HOST ? cudaFreeHost(p) : cudaFree(p)) != cudaSuccess) (void)cudaGetLastError();
+}
+}  // namespace
+
+// (never destroyed: the CUDA context may be gone before static destructors run)
+BlockCache& block_cache(bool host) {
+    static BlockCache* dev = new BlockCache(alloc_block<false>, free_block<false>, (size_t)4 << 30);
+    static BlockCache* pinned = new BlockCache(alloc_block<true>, free_block<true>, (size_t)256 << 20);
+    return host ? *pinned : *dev;
+}
 
 int set_error(int code, const std::string& msg) {
     g_last_error = msg;
@@ -1373,15 +1288,16 @@ int run_adjoint(rms_sim* s, const rms_run_opts* o, const double* g_sigw, rms_adj
         const long long mb = std::atoll(cap);
         if (mb > 0) budget = std::min<size_t>(budget, (size_t)mb << 20);
     }
-    // half the free memory, asked for when the records are large or do not fit:
-    // cudaMemGetInfo waits for the whole machine's memory calls (0.1 to 20 ms)
-    auto half_free = [] {
+    // half the free memory, the block cache's counted in, asked for when the records
+    // are large or do not fit: cudaMemGetInfo waits for the whole machine's memory
+    // calls (0.1 to 20 ms)
+    auto half_free = [device] {
         size_t mfree = 0, mtotal = 0;
         if (cudaMemGetInfo(&mfree, &mtotal) != cudaSuccess) {
             (void)cudaGetLastError();
             mfree = 0;
         }
-        return mfree / 2;
+        return (mfree + block_cache(false).held(device)) / 2;
     };
     const char* genv = std::getenv("RMS_ADJOINT_GROUPED");
     int64_t chunk = 0;
@@ -1988,6 +1904,13 @@ void rms_sim_destroy(rms_sim* s) {
     if (!s) return;
     delete s->dev;
     delete s;
+}
+
+int rms_memory_trim(size_t* device_bytes, size_t* host_bytes) {
+    const size_t d = block_cache(false).trim(), h = block_cache(true).trim();
+    if (device_bytes) *device_bytes = d;
+    if (host_bytes) *host_bytes = h;
+    return RMS_OK;
 }
 
 int rms_rng_doubles(uint64_t seed, uint64_t walker, int n, double* out) {

@@ -48,10 +48,9 @@
 
 #include <algorithm>
 #include <mutex>
-#include <new>
-#include <vector>
 
 #include "../../include/rms.h"
+#include "block_cache.h"
 #include "rms_internal.h"
 
 namespace rms {
@@ -835,64 +834,25 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// A call's workspace: packed waveforms and the error word on the device, and a
-// pinned word to read the latter into.  Calls of several threads or streams each
-// take their own; at most kMostFree wait for the next ones.
+// A call's workspace, from the library's block cache: packed waveforms and the
+// error word on the device, and a pinned word to read the latter into.  Calls of
+// several threads or streams each take their own; it goes back when the stream has
+// been waited for (`idle`: it has).
 struct Workspace {
+    cudaStream_t st;
+    int device;
     void* p = nullptr;
-    size_t bytes = 0;
-    int* herr = nullptr;
-    int device = -1;
-};
-std::mutex g_ws_mu;
-std::vector<Workspace> g_ws_free;
-constexpr size_t kMostFree = 4;
-
-void free_workspace(const Workspace& w) {
-    if (w.p) cudaFree(w.p);   // waits for the device
-    if (w.herr) cudaFreeHost(w.herr);
-}
-
-bool take_workspace(size_t bytes, int device, Workspace& w) {
-    {
-        std::lock_guard<std::mutex> lk(g_ws_mu);
-        int pick = -1;   // one that is large enough, else any (it is grown)
-        for (int k = 0; k < (int)g_ws_free.size(); ++k)
-            if (g_ws_free[k].device == device && (pick < 0 || g_ws_free[k].bytes >= bytes)) pick = k;
-        if (pick >= 0) {
-            w = g_ws_free[pick];
-            g_ws_free.erase(g_ws_free.begin() + pick);
-        }
+    void* herr = nullptr;
+    size_t n = 0, nh = 0;
+    bool idle = true;
+    bool take(size_t bytes) {
+        return block_cache(false).take(bytes, device, &p, &n) == 0 &&
+               block_cache(true).take(sizeof(int), device, &herr, &nh) == 0;
     }
-    if (w.p && w.bytes >= bytes) return true;
-    free_workspace(w);
-    w = Workspace{};
-    w.device = device;
-    w.bytes = bytes;
-    if (cudaMalloc(&w.p, bytes) == cudaSuccess && cudaMallocHost(reinterpret_cast<void**>(&w.herr), sizeof(int)) == cudaSuccess)
-        return true;
-    free_workspace(w);
-    w = Workspace{};
-    return false;
-}
-
-// Returns a call's workspace; `idle`: the stream has been waited for.
-struct WorkspaceGuard {
-    Workspace w;
-    bool idle = false;
-    ~WorkspaceGuard() {
-        if (!w.p) return;
-        if (idle) {
-            std::lock_guard<std::mutex> lk(g_ws_mu);
-            if (g_ws_free.size() < kMostFree) {
-                try {
-                    g_ws_free.push_back(w);
-                    return;
-                } catch (const std::bad_alloc&) {
-                }
-            }
-        }
-        free_workspace(w);
+    ~Workspace() {
+        if (!idle && cudaStreamSynchronize(st) != cudaSuccess) (void)cudaGetLastError();
+        if (p) block_cache(false).give(p, n, device);
+        if (herr) block_cache(true).give(herr, nh, device);
     }
 };
 
@@ -972,9 +932,10 @@ int contract_phases(const float* d_pos, int64_t nwalk, int nbins, const float* d
         const int n_mpairs = (nwave + 2 * kTileM - 1) / (2 * kTileM);
         const int n_mtiles = 2 * n_mpairs;   // the last tiles' rows past nwave are zero
         const size_t gbytes = (size_t)n_mtiles * nk * 2 * kGBytes;
-        WorkspaceGuard ws;
-        if (!take_workspace(gbytes + 256, dev, ws.w)) return fail(RMS_ERR_NOMEM, "workspace");
-        uint8_t* gpack = static_cast<uint8_t*>(ws.w.p);
+        Workspace ws{st, dev};
+        if (!ws.take(gbytes + 256)) return fail(RMS_ERR_NOMEM, "workspace");
+        ws.idle = false;
+        uint8_t* gpack = static_cast<uint8_t*>(ws.p);
         int* d_err = reinterpret_cast<int*>(gpack + gbytes);
         const int64_t items = (int64_t)n_mtiles * kTileM * nk * (kKc / 8);
         pack_waves_kernel<<<(unsigned)std::min<int64_t>(1024, (items + 255) / 256), 256, 0, st>>>(
@@ -1025,11 +986,11 @@ int contract_phases(const float* d_pos, int64_t nwalk, int nbins, const float* d
         });
         if (ev.b) cudaEventRecord(ev.b, st);
         if (cudaGetLastError() != cudaSuccess) return fail(RMS_ERR_CUDA, "tensor-core contraction launch");
-        if (cudaMemcpyAsync(ws.w.herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        if (cudaMemcpyAsync(ws.herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
             return fail(RMS_ERR_CUDA, "tensor-core contraction");
         ws.idle = true;
-        if (*ws.w.herr & kErrTimeout) return fail(RMS_ERR_TIMEOUT, "a pipeline wait of the tensor-core contraction ran out");
+        if (*static_cast<const int*>(ws.herr) & kErrTimeout) return fail(RMS_ERR_TIMEOUT, "a pipeline wait of the tensor-core contraction ran out");
     }
     if (kernel_ms && (cudaEventElapsedTime(kernel_ms, ev.a, ev.b) != cudaSuccess))
         return fail(RMS_ERR_CUDA, "contraction timing");

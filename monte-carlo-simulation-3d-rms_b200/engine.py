@@ -30,7 +30,7 @@ ERRORS = {-1: "ARG", -2: "IO", -3: "FORMAT", -4: "RANGE", -5: "CUDA", -6: "NOMEM
 EXPORTS = ("rms_sim_create", "rms_sim_load_dir", "rms_sim_set_lattice", "rms_sim_run",
            "rms_sim_field_size", "rms_sim_get", "rms_sim_get_trace", "rms_sim_get_trace_positions",
            "rms_sim_write_dir",
-           "rms_sim_last_timing", "rms_batch_run", "rms_last_error", "rms_sim_destroy",
+           "rms_sim_last_timing", "rms_batch_run", "rms_last_error", "rms_sim_destroy", "rms_memory_trim",
            "rms_rng_doubles", "rms_rng_floats", "rms_philox4x32_10", "rms_version",
            "rms_split_variant", "rms_rng_split", "rms_sim_run_noalloc", "rms_contract_phases",
            "rms_adjoint_run", "rms_adjoint_jacobian", "rms_autotune", "rms_batch_graph_create", "rms_graph_run", "rms_graph_destroy",
@@ -122,6 +122,7 @@ def lib():
         L.rms_sim_last_timing.argtypes = [C.c_void_p, _DP, _DP]
         L.rms_batch_run.argtypes = [C.POINTER(C.c_void_p), C.c_int, C.POINTER(RunOpts)]
         L.rms_sim_destroy.argtypes = [C.c_void_p]
+        L.rms_memory_trim.argtypes = [C.POINTER(C.c_size_t)] * 2
         L.rms_rng_doubles.argtypes = [C.c_uint64, C.c_uint64, C.c_int, _DP]
         L.rms_rng_floats.argtypes = [C.c_uint64, C.c_uint64, C.c_int, C.POINTER(C.c_float)]
         L.rms_philox4x32_10.argtypes = [C.POINTER(C.c_uint32)] * 3
@@ -413,6 +414,15 @@ def batch_run(sims, seed: int = 0, precision: str = "compat", device: int = 0, s
     arr = (C.c_void_p * len(sims))(*[s._h.value for s in sims])
     opts = _opts(seed, precision, device, stream, variant=variant, shard=shard)
     _check(lib().rms_batch_run(arr, len(sims), C.byref(opts)))
+
+
+def trim_memory() -> tuple:
+    """Give back the device and pinned memory the library keeps of closed
+    simulations and finished contractions (for a program that wants it for
+    something else); returns the bytes of each."""
+    d, h = C.c_size_t(), C.c_size_t()
+    _check(lib().rms_memory_trim(C.byref(d), C.byref(h)))
+    return d.value, h.value
 
 
 def contract_phases(d_pos: int, nwalk: int, nbins: int, d_wave: int, nwave: int, d_out: int,
