@@ -525,11 +525,15 @@ int prepare_lattice(rms_sim* s, cudaStream_t st, bool split, int bits) {
     return RMS_OK;
 }
 
-// Row sets of an axon walked by `warps` warps at once (a row set is row_sz
-// doubles): warps of one row set add into the same addresses at about the same
-// time, so one set per 64 warps, at most 16, and no more than 256 MB of them.
-int split_row_sets(int64_t warps, size_t row_sz) {
-    const int64_t fit = std::max<int64_t>(1, (int64_t)(((size_t)256 << 20) / (row_sz * sizeof(double))));
+// Row sets of one of a launch's naxons axons, walked by `warps` warps at once (a
+// row set is row_sz doubles): warps of one row set add into the same addresses at
+// about the same time, so one set per 64 warps, at most 16, and no more than 256 MB
+// of them -- nor than the axon's part of 1 GB, since a launch clears and reads back
+// the sets of all its axons, of which it walks one or two at a time.  (One set
+// each whatever its size: the results themselves.)
+int split_row_sets(int64_t warps, size_t row_sz, int naxons) {
+    const size_t most = std::min<size_t>((size_t)256 << 20, ((size_t)1 << 30) / naxons);
+    const int64_t fit = std::max<int64_t>(1, (int64_t)(most / (row_sz * sizeof(double))));
     return (int)std::max<int64_t>(1, std::min<int64_t>({warps / 64, 16, fit}));
 }
 
@@ -733,7 +737,7 @@ int plan_launch(std::vector<LaunchJob>& jobs, const rms_run_opts* o, LaunchPlan&
             AxonDesc& x = p.axons[k];
             fill_axon_desc(x, jobs[k].s, jobs[k].w0, jobs[k].w1, tile_begin[k], jobs[k].seed,
                            jobs[k].s->dev->packed(lattice_bits).as<uint8_t>());
-            x.ncopy = split_row_sets(std::min<int64_t>(tile_begin[k + 1] - tile_begin[k], nwarps), row_sz);
+            x.ncopy = split_row_sets(std::min<int64_t>(tile_begin[k + 1] - tile_begin[k], nwarps), row_sz, naxons);
             x.row_off = (int64_t)nsets;
             nsets += (size_t)x.ncopy * row_sz;
         }
