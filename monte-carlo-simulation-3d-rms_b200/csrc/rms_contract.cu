@@ -51,6 +51,7 @@
 
 #include "../../include/rms.h"
 #include "block_cache.h"
+#include "once_per_device.h"
 #include "rms_internal.h"
 
 namespace rms {
@@ -942,19 +943,19 @@ int contract_phases(const float* d_pos, int64_t nwalk, int nbins, const float* d
             d_wave, nwave, K, nk, n_mtiles, gpack, d_err, d_out);
         if (cudaGetLastError() != cudaSuccess) return fail(RMS_ERR_CUDA, "waveform packing launch");
 
-        static std::once_flag attr_once;
-        static cudaError_t attr_err = cudaSuccess;
-        std::call_once(attr_once, [] {
+        static OncePerDevice opt_in;
+        const int attr_err = opt_in(dev, [] {
+            cudaError_t e = cudaSuccess;
             for (int tn : {64, 128, 256, 257})   // (257: 256 with full pairs)
                 by_tile(tn, tn == 257, [&]<int TN, bool PAIRS>() {
                     for (const void* k : {(const void*)contract_tc_kernel<TN, PAIRS>,
                                           (const void*)contract_presplit_kernel<TN, PAIRS>})
-                        if (attr_err == cudaSuccess)
-                            attr_err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                            (int)kSmemBytes);
+                        if (e == cudaSuccess)
+                            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
                 });
+            return e;
         });
-        if (attr_err != cudaSuccess) return fail(RMS_ERR_CUDA, "shared memory attribute");
+        if (attr_err) return fail(RMS_ERR_CUDA, "shared memory attribute");
         const int tn = walkers_per_tile(nwalk, n_mpairs, sms);
         CUtensorMap mhi, mlo;
         if (presplit) {
