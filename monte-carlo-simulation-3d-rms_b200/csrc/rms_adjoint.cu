@@ -166,7 +166,7 @@ struct LaneArr {
 // read back are not kept (28 KB a block in FORM 1, 12 / 20 KB in FORM 2, where
 // all forms once held 25-33 KB), and the waveform tables are fetched into
 // shared memory while the bin is walked.  With that FORM 1 runs 6 blocks (80
-// registers, 16 bytes spilled) and FORM 2 5 (96 registers, none); 7 or 8 blocks
+// registers, 24 bytes spilled, 32 in the Jacobian form) and FORM 2 5 (96 registers, none); 7 or 8 blocks
 // spill and take the L1.  FORM 0: 5 for the weighted loss, the compiler's choice
 // for the Jacobian.
 // Measured on a 64x64x512 axon, 5000 steps, 1000 bins, 16 waveforms (weighted /

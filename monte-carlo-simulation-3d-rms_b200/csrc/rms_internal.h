@@ -20,8 +20,8 @@ constexpr int kErrStep = 2;                     // a segment found no face (step
 constexpr int kErrTimeout = 4;                  // a bounded wait of a pipelined kernel ran out
 
 // One simulation ("axon") of a split-precision launch.  A launch walks the
-// tiles (32 walkers) of all its axons; axon k owns global tiles
-// [tile_begin, tile_begin + ceil((walker_end - walker_begin) / 32)).
+// tiles (WalkArgs::tile_w walkers, at most 32) of all its axons; axon k owns global
+// tiles [tile_begin, tile_begin + ceil((walker_end - walker_begin) / tile_w)).
 struct AxonDesc {
     const uint8_t* lat;         // padded, packed lattice of this axon
     int n1, n2, n3, nc;

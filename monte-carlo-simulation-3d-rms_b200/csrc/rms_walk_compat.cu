@@ -8,16 +8,17 @@
 // sum is rounded like the reference's own expressions.
 //
 // What differs from the reference, by design:
-//  - cross-walker sums: warp shuffles into per-warp FP64 rows, then one
-//    ordered reduction (no CAS atomics, repeatable);
+//  - cross-walker sums: records staged in shared memory and added up in batches,
+//    by a lane per group of columns or per b-value, into per-warp FP64 rows, then
+//    one ordered reduction (no CAS atomics, repeatable);
 //  - PGSE phase: per walker the displacement sums over each gradient's two
 //    lobes are formed from running prefix sums at the lobe edges, instead of
 //    an O(Ngrad) update every step into a 16 KB local array
 //    (main_PGSE.cu:99-100, 340-346).  phase_j = |g| (g_hat . V_j) dt with
 //    V_j = sum_{lobe 1} dx - sum_{lobe 2} dx is the same sum, reassociated;
 //  - walls: periodic as an option beside the reference's mirror;
-//  - persistent grid: each warp walks 32 walkers at a time, tiles strided by
-//    the number of warps in the grid.
+//  - persistent grid: each warp walks a tile of walkers at a time, 32 or fewer
+//    (tile_width in rms_api.cpp), tiles strided by the number of warps in the grid.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -186,9 +187,9 @@ __device__ __noinline__ void add_pgse(const WalkArgs& a, int nthr, int t0, doubl
 // exact quotients of all three.  Every value that reaches the walker is the
 // reference's expression, rounded as written.
 //
-// MINB, resident blocks per SM: 4 (113 registers), 5 (96, 24 bytes spilled) or 6
-// (80, 156 bytes); the launch takes the one whose rounds of tiles end first
-// (compat_form in rms_api.cpp).
+// MINB, resident blocks per SM: 4 (narrow pulses 108 registers, PGSE 119), 5 (96, 32
+// and 68 bytes spilled) or 6 (80, 156 and 176 bytes); the launch takes the one whose
+// rounds of tiles end first (compat_form in rms_api.cpp).
 template <int NCMAX, bool TRACE, bool PGSE, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) walk_compat_kernel(const __grid_constant__ WalkArgs a) {
     __shared__ double s_step[NCMAX], s_rstep[NCMAX], s_t2[NCMAX], s_rt2[NCMAX], s_pij[NCMAX * NCMAX];

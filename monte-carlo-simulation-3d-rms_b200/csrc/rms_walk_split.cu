@@ -195,8 +195,9 @@ __device__ __noinline__ void wave_final(const double* ph, int nthr, int nwave, d
 // warp-record costs five loads, 24 conversions and adds and ~30 paired products
 // (__fmul2_rn: two walkers an instruction), no shuffle.  1e6 walkers x 2000
 // steps on a 128x128x900 axon, walk kernel: 12.5 / 35.6 ms with 100 / 2000
-// records before, 10.4 / 25.3 ms now (12.3 / 27.1 with the step of that day).  KR = 8 up to 256 threads a block (4.2 KB
-// of staging per warp), 4 above, so the static shared memory stays under 48 KB.
+// records one at a time, 12.3 / 27.1 in batches; 10.4 / 25.3 ms since the step
+// itself is shorter (split_step.cuh).  KR = 8 up to 256 threads a block (4.2 KB of
+// staging per warp), 4 above, so the static shared memory stays under 48 KB.
 __host__ __device__ constexpr int rec_batch(int block) { return block <= 256 ? 8 : 4; }
 constexpr int kStageRow = 4 * 32 + 4;   // floats of a staged record: x, y, z, s0 of 32 walkers, and 4 of padding
 constexpr int kStageOnes = -4;          // before the first record, four ones

@@ -2,10 +2,10 @@
 //
 // The reference adds every walker's record into the same global addresses
 // with an FP64 compare-and-swap loop (hpc_code/lib/main.cu:40-56, 344-378):
-// 23+Nbvec contended atomics per walker per record.  Here a warp first sums
-// its 32 walkers with register shuffles, in a fixed order, and one lane per
-// value adds the warp total into that warp's private accumulator row -- no
-// atomics, and a repeatable result for a fixed launch shape.
+// 23+Nbvec contended atomics per walker per record.  Here a warp first sums its
+// walkers: a final sum by register shuffles in a fixed order, records and signals
+// by lanes that each add up a column, b-value or gradient over the walkers
+// (signal_lanes), and one lane per value passes the warp's sum on.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -103,6 +103,7 @@ def test_rules(tmp_path):
     assert out.returncode == 0 and out.stdout == "ok\n", out.stderr
 
 
-def test_trim_without_a_device():
+def test_trim_leaves_nothing():
     from rms_b200 import engine
+    engine.trim_memory()
     assert engine.trim_memory() == (0, 0)
